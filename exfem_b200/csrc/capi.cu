@@ -103,7 +103,11 @@ static int set_material(exfem_block_s* b, const exfem_material* m) {
     for (int i = 0; i < m->ntab; ++i) {
       d.ep[i] = m->ep_tab[i];
       d.sy[i] = m->sy_tab[i];
+      const double dx = i ? d.ep[i] - d.ep[i - 1] : 0.0;
+      d.slope[i] = fabs(dx) <= 4.930380657631324e-32 ? 0.0 : (d.sy[i] - d.sy[i - 1]) / dx;  // spacing(eps) of float64
+      d.rh[i] = 1.0 / (3.0 * d.mu + d.Hk + d.slope[i]);
     }
+    d.rh0 = 1.0 / (3.0 * d.mu + d.Hk);
   }
   return EXFEM_OK;
 }
