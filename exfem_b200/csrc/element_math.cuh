@@ -137,6 +137,33 @@ __host__ __device__ constexpr double tet10_dN(int g, int a, int i) {
                         tet_L(g, tet_edge(a - 4, 0)) * tet_dL(tet_edge(a - 4, 1), i));
 }
 
+// ---------------------------------------------------------------- shape-function gradients
+// dN_b / dxi_i of the trilinear hexahedron at corner-ordered Gauss point g
+__device__ __forceinline__ double hex_dN(int g, int b, int i) {
+  const double p0 = HEX_GQ * hex_sign(g, 0), p1 = HEX_GQ * hex_sign(g, 1), p2 = HEX_GQ * hex_sign(g, 2);
+  const double s0 = hex_sign(b, 0), s1 = hex_sign(b, 1), s2 = hex_sign(b, 2);
+  const double f0 = 1.0 + s0 * p0, f1 = 1.0 + s1 * p1, f2 = 1.0 + s2 * p2;
+  return i == 0 ? 0.125 * s0 * f1 * f2 : (i == 1 ? 0.125 * f0 * s1 * f2 : 0.125 * f0 * f1 * s2);
+}
+
+template <class T>
+__device__ __forceinline__ void matmul3(const T (&A)[9], const T (&B)[9], T (&C)[9]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) C[3 * i + j] = A[3 * i] * B[j] + A[3 * i + 1] * B[3 + j] + A[3 * i + 2] * B[6 + j];
+}
+
+__device__ __forceinline__ double elem_dN(int et, int g, int a, int i) {
+  if (et == EXFEM_C3D8) return hex_dN(g, a, i);
+  switch (g) {
+    case 0: return tet10_dN(0, a, i);
+    case 1: return tet10_dN(1, a, i);
+    case 2: return tet10_dN(2, a, i);
+    default: return tet10_dN(3, a, i);
+  }
+}
+
 // ---------------------------------------------------------------- tile-major streams
 // Per-element streams of the matrix-free operator (geometry, J2 tangent data) are
 // stored tile-major ("AoSoA") over the block's tile order: tiles of `tile`

@@ -12,22 +12,6 @@
 
 namespace exfem {
 
-// dN_b / dxi_i of the trilinear hexahedron at corner-ordered Gauss point g
-__device__ __forceinline__ double hex_dN(int g, int b, int i) {
-  const double p0 = HEX_GQ * hex_sign(g, 0), p1 = HEX_GQ * hex_sign(g, 1), p2 = HEX_GQ * hex_sign(g, 2);
-  const double s0 = hex_sign(b, 0), s1 = hex_sign(b, 1), s2 = hex_sign(b, 2);
-  const double f0 = 1.0 + s0 * p0, f1 = 1.0 + s1 * p1, f2 = 1.0 + s2 * p2;
-  return i == 0 ? 0.125 * s0 * f1 * f2 : (i == 1 ? 0.125 * f0 * s1 * f2 : 0.125 * f0 * f1 * s2);
-}
-
-template <class T>
-__device__ __forceinline__ void matmul3(const T (&A)[9], const T (&B)[9], T (&C)[9]) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) C[3 * i + j] = A[3 * i] * B[j] + A[3 * i + 1] * B[3 + j] + A[3 * i + 2] * B[6 + j];
-}
-
 // Q = C * iJ^T for symmetric C given as 6 components, scaled by w
 template <class T>
 __device__ __forceinline__ void cotangent(const T (&c)[6], T w, const T (&iJ)[9], T (&Q)[9]) {
@@ -414,210 +398,6 @@ int build_geometry(exfem_block_s* b) {
   // the legacy stream only: a device-wide synchronisation would invalidate a graph
   // capture in progress on another host thread
   EX_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
-  return EXFEM_OK;
-}
-
-// ---------------------------------------------------------------- element tangents
-__device__ __forceinline__ double elem_dN(int et, int g, int a, int i) {
-  if (et == EXFEM_C3D8) return hex_dN(g, a, i);
-  switch (g) {
-    case 0: return tet10_dN(0, a, i);
-    case 1: return tet10_dN(1, a, i);
-    case 2: return tet10_dN(2, a, i);
-    default: return tet10_dN(3, a, i);
-  }
-}
-
-template <class OutT>
-__device__ __forceinline__ void store_out(OutT* p, double v);
-template <> __device__ __forceinline__ void store_out<double>(double* p, double v) { *p = v; }
-template <> __device__ __forceinline__ void store_out<float>(float* p, double v) { *p = (float)v; }
-template <> __device__ __forceinline__ void store_out<__nv_bfloat16>(__nv_bfloat16* p, double v) {
-  *p = __float2bfloat16((float)v);
-}
-
-// One block = EPB elements x NN threads.  Phase 1: one thread per Gauss point
-// computes the inverse Jacobian, weighted volume and material tangent data into
-// shared memory.  Phase 2: one thread per element node a computes the three rows
-// 3a..3a+2 of Ke = sum_g w_g dF_a : C_g : dF_b (the reference's G^T A G).
-template <int ET, int MODE, class OutT>
-__global__ void __launch_bounds__(64)
-stiffness_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict__ conn,
-                 const double* __restrict__ u, const double* __restrict__ scale,
-                 const double* __restrict__ st_old, const double* __restrict__ tan_in,
-                 const MatDev mat, const double* __restrict__ lam_e, const double* __restrict__ mu_e,
-                 OutT* __restrict__ Ke, double* __restrict__ ediag, const int32_t* __restrict__ tpos, int tile) {
-  using Tr = ElemTraits<ET>;
-  constexpr int NN = Tr::nnode, NG = Tr::ngp, ND = 3 * NN, EPB = 64 / NN;
-  constexpr bool BBAR = ET == EXFEM_C3D8;
-  __shared__ double s_iJ[EPB][NG][9];
-  __shared__ double s_vol[EPB][NG];
-  __shared__ double s_tn[EPB][NG][8];
-  __shared__ double s_iJ0[EPB][9];
-  const int le = threadIdx.x / NN, a = threadIdx.x % NN;
-  const int64_t e = (int64_t)blockIdx.x * EPB + le;
-  const bool valid = le < EPB && e < ne;
-  const bool own = valid && lam_e;  // per-element Lame parameters override the material's
-  const double lam_k = own ? lam_e[e] : mat.lam, mu_k = own ? mu_e[e] : mat.mu;
-  const int ns = mat.kind == EXFEM_J2 ? 19 : 1;
-  if (valid && a < NG) {
-    const int g = a;
-    const double sc = scale ? scale[e] : 1.0;
-    double J[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    double J0[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, G0[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int b = 0; b < NN; ++b) {
-      const int64_t n3 = 3 * (int64_t)conn[e * NN + b];
-      for (int i = 0; i < 3; ++i) {
-        const double dn = elem_dN(ET, g, b, i);
-        const double dn0 = BBAR ? 0.125 * hex_sign(b, i) : 0.0;
-        for (int c = 0; c < 3; ++c) {
-          const double xv = X[n3 + c], uv = u ? u[n3 + c] : 0.0;
-          J[3 * c + i] += xv * dn;
-          G[3 * c + i] += uv * dn;
-          if (BBAR) {
-            J0[3 * c + i] += xv * dn0;
-            G0[3 * c + i] += uv * dn0;
-          }
-        }
-      }
-    }
-    double iJ[9], H[9];
-    const double detJ = inv3(J, iJ);
-    matmul3(G, iJ, H);
-    if (BBAR) {
-      double iJ0[9], H0[9];
-      inv3(J0, iJ0);
-      matmul3(G0, iJ0, H0);
-      const double bb = ((H0[0] + H0[4] + H0[8]) - (H[0] + H[4] + H[8])) / 3.0;
-      H[0] += bb;
-      H[4] += bb;
-      H[8] += bb;
-      if (g == 0)
-        for (int k = 0; k < 9; ++k) s_iJ0[le][k] = iJ0[k];
-    }
-    double zero_state[19];
-    for (int k = 0; k < 19; ++k) zero_state[k] = 0.0;
-    const double* st = st_old ? st_old + (e * NG + g) * ns : zero_state;
-    double sig[6], tn[8];
-    if (tan_in) {
-      for (int k = 0; k < 8; ++k) tn[k] = tan_in[tile_index(tpos[e], g * 8 + k, NG * 8, tile)];
-    } else {
-      material_stress(mat, lam_k, mu_k, H, st, nullptr, sig, tn);
-    }
-    for (int k = 0; k < 9; ++k) s_iJ[le][g][k] = iJ[k];
-    s_vol[le][g] = (ET == EXFEM_C3D8 ? 1.0 : 1.0 / 24.0) * detJ * sc;
-    for (int k = 0; k < 8; ++k) s_tn[le][g][k] = tn[k];
-  }
-  __syncthreads();
-  if (!valid) return;
-  double dNa[NG][3], dN0a[3] = {0, 0, 0};
-#pragma unroll
-  for (int g = 0; g < NG; ++g)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      double s = 0.0;
-#pragma unroll
-      for (int i = 0; i < 3; ++i) s += elem_dN(ET, g, a, i) * s_iJ[le][g][3 * i + j];
-      dNa[g][j] = s;
-    }
-  if (BBAR)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      double s = 0.0;
-#pragma unroll
-      for (int i = 0; i < 3; ++i) s += 0.125 * hex_sign(a, i) * s_iJ0[le][3 * i + j];
-      dN0a[j] = s;
-    }
-  const double Kb = own ? lam_k + 2.0 * mu_k / 3.0 : mat.K, mu = mu_k;
-  for (int b = (MODE == 1 ? a : 0); b < (MODE == 1 ? a + 1 : NN); ++b) {
-    double dNb[NG][3], dN0b[3] = {0, 0, 0};
-#pragma unroll
-    for (int g = 0; g < NG; ++g)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        double s = 0.0;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) s += elem_dN(ET, g, b, i) * s_iJ[le][g][3 * i + j];
-        dNb[g][j] = s;
-      }
-    if (BBAR)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        double s = 0.0;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) s += 0.125 * hex_sign(b, i) * s_iJ0[le][3 * i + j];
-        dN0b[j] = s;
-      }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      double acc[3] = {0, 0, 0};
-#pragma unroll
-      for (int g = 0; g < NG; ++g) {
-        double H[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        H[3 * k + 0] = dNb[g][0];
-        H[3 * k + 1] = dNb[g][1];
-        H[3 * k + 2] = dNb[g][2];
-        if (BBAR) {
-          const double bb = (dN0b[k] - dNb[g][k]) / 3.0;
-          H[0] += bb;
-          H[4] += bb;
-          H[8] += bb;
-        }
-        double de[6], ds[6];
-        sym_from_grad(H, de);
-        tangent_stress(Kb, mu, s_tn[le][g], de, ds);
-        const double trs = ds[0] + ds[1] + ds[2];
-        const double rows[3][3] = {{ds[0], ds[3], ds[5]}, {ds[3], ds[1], ds[4]}, {ds[5], ds[4], ds[2]}};
-        const double w = s_vol[le][g];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          double v = rows[i][0] * dNa[g][0] + rows[i][1] * dNa[g][1] + rows[i][2] * dNa[g][2];
-          if (BBAR) v += (dN0a[i] - dNa[g][i]) / 3.0 * trs;
-          acc[i] += w * v;
-        }
-      }
-      if (MODE == 0) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) store_out(Ke + e * ND * ND + (3 * a + i) * ND + 3 * b + k, acc[i]);
-      } else {
-        ediag[(e * NN + a) * 3 + k] = acc[k];
-      }
-    }
-  }
-}
-
-template <int ET, class OutT>
-static void stiffness_go(exfem_block_s* b, const double* u, const double* st_old, const double* tan_in,
-                         OutT* Ke, double* ediag, cudaStream_t s) {
-  constexpr int EPB = 64 / ElemTraits<ET>::nnode;
-  const unsigned grid = (unsigned)((b->ne + EPB - 1) / EPB);
-  if (ediag)
-    stiffness_kernel<ET, 1, OutT><<<grid, 64, 0, s>>>(b->ne, b->X.p, b->conn.p, u, b->scale.p, st_old,
-                                                      tan_in, b->mat, b->lam_e.p, b->mu_e.p, Ke, ediag,
-                                                      b->tpos.p, b->tile);
-  else
-    stiffness_kernel<ET, 0, OutT><<<grid, 64, 0, s>>>(b->ne, b->X.p, b->conn.p, u, b->scale.p, st_old,
-                                                      tan_in, b->mat, b->lam_e.p, b->mu_e.p, Ke, ediag,
-                                                      b->tpos.p, b->tile);
-}
-
-int launch_stiffness(exfem_block_s* b, const double* u, const double* st_old, int dtype, void* Ke,
-                     double* ediag, cudaStream_t s, const double* tan_in) {
-  if (b->ne == 0) return EXFEM_OK;
-  if (dtype == EXFEM_F64) {
-    if (b->etype == EXFEM_C3D8) stiffness_go<EXFEM_C3D8>(b, u, st_old, tan_in, (double*)Ke, ediag, s);
-    else stiffness_go<EXFEM_C3D10>(b, u, st_old, tan_in, (double*)Ke, ediag, s);
-  } else if (dtype == EXFEM_F32) {
-    if (b->etype == EXFEM_C3D8) stiffness_go<EXFEM_C3D8>(b, u, st_old, tan_in, (float*)Ke, ediag, s);
-    else stiffness_go<EXFEM_C3D10>(b, u, st_old, tan_in, (float*)Ke, ediag, s);
-  } else if (dtype == EXFEM_BF16) {
-    if (b->etype == EXFEM_C3D8) stiffness_go<EXFEM_C3D8>(b, u, st_old, tan_in, (__nv_bfloat16*)Ke, ediag, s);
-    else stiffness_go<EXFEM_C3D10>(b, u, st_old, tan_in, (__nv_bfloat16*)Ke, ediag, s);
-  } else {
-    set_error("unsupported Ke dtype %d", dtype);
-    return EXFEM_ERR_ARG;
-  }
-  EX_LAUNCH_CHECK();
   return EXFEM_OK;
 }
 
