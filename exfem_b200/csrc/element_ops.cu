@@ -1,258 +1,12 @@
-// FP64 element kernels: internal force with the J2 return map (and the
-// per-Gauss-point consistent-tangent data it produces), element tangents Ke,
-// element-averaged stresses, deterministic assembly (gather plan or colour
-// scatter), and the stored-Ke element-by-element product.
+// FP64 element operations: deterministic assembly of element vectors (gather plan or
+// colour scatter), the geometry streams of the matrix-free operator, initial-stress
+// stiffness, and the stored-Ke element-by-element product and diagonals.
 //
-// Reference: gfem/model.py:35-111 (geom, B-bar defgrad, force, stiff),
-// 129-137 (cauchy), 162-173 (ops_matvec / ops_diagonal), 241-267 (gather plan
-// assembly), 466-486 (Model.internal_force / element_stiffness).
-#include <cuda_bf16.h>
-
+// Reference: gfem/model.py:113-117 (geo_stiff), 162-173 (ops_matvec / ops_diagonal),
+// 241-267 (gather plan assembly), 466-486 (Model.internal_force / element_stiffness).
 #include "internal.h"
 
 namespace exfem {
-
-// Q = C * iJ^T for symmetric C given as 6 components, scaled by w
-template <class T>
-__device__ __forceinline__ void cotangent(const T (&c)[6], T w, const T (&iJ)[9], T (&Q)[9]) {
-  const T r[3][3] = {{c[0], c[3], c[5]}, {c[3], c[1], c[4]}, {c[5], c[4], c[2]}};
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-      Q[3 * i + k] = w * (r[i][0] * iJ[3 * k] + r[i][1] * iJ[3 * k + 1] + r[i][2] * iJ[3 * k + 2]);
-}
-
-// ---------------------------------------------------------------- force / tangent / stress
-template <int ET, int MODE>
-__global__ void __launch_bounds__(128)
-force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict__ conn,
-             const double* __restrict__ u, const double* __restrict__ scale,
-             const double* __restrict__ st_old, double* __restrict__ st_new, double* __restrict__ fe,
-             double* __restrict__ tan64, float* __restrict__ tan32, double* __restrict__ S,
-             double* __restrict__ mises, double* __restrict__ peeq, const MatDev mat,
-             const double* __restrict__ lam_e, const double* __restrict__ mu_e,
-             const int32_t* __restrict__ tpos, int tile) {
-  using Tr = ElemTraits<ET>;
-  constexpr int NN = Tr::nnode, NG = Tr::ngp;
-  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e >= ne) return;
-  // per-element Lame parameters (linear elasticity) override the material's
-  const double lam_k = lam_e ? lam_e[e] : mat.lam, mu_k = lam_e ? mu_e[e] : mat.mu;
-  const int ns = mat.kind == EXFEM_J2 ? 19 : 1;
-  const double sc = (MODE != FORCE_STRESS && scale) ? scale[e] : 1.0;
-  int nod[NN];
-#pragma unroll
-  for (int a = 0; a < NN; ++a) nod[a] = conn[e * NN + a];
-  double Sacc[6] = {0, 0, 0, 0, 0, 0}, vsum = 0.0, pacc = 0.0;
-  const double* st_e = st_old ? st_old + e * (int64_t)NG * ns : nullptr;
-  double* sn_e = (MODE == FORCE_FULL && st_new) ? st_new + e * (int64_t)NG * ns : nullptr;
-  double zero_state[19];
-#pragma unroll
-  for (int k = 0; k < 19; ++k) zero_state[k] = 0.0;
-
-  if constexpr (ET == EXFEM_C3D8) {
-    double xa[8][3], ua[8][3], cm[7][3], um[7][3];
-#pragma unroll
-    for (int a = 0; a < 8; ++a)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        xa[a][c] = X[3 * (int64_t)nod[a] + c];
-        ua[a][c] = u[3 * (int64_t)nod[a] + c];
-      }
-    hex_to_modal(xa, cm);
-    hex_to_modal(ua, um);
-    double J0[9], iJ0[9], G0[9], H0[9];
-#pragma unroll
-    for (int n = 0; n < 3; ++n)
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        J0[3 * n + i] = cm[i][n];
-        G0[3 * n + i] = um[i][n];
-      }
-    inv3(J0, iJ0);
-    matmul3(G0, iJ0, H0);
-    const double tr0 = H0[0] + H0[4] + H0[8];
-    double Fm[7][3];
-#pragma unroll
-    for (int k = 0; k < 7; ++k) Fm[k][0] = Fm[k][1] = Fm[k][2] = 0.0;
-    double tacc = 0.0;
-#pragma unroll 1
-    for (int g = 0; g < 8; ++g) {
-      const double x = HEX_GQ * hex_sign(g, 0), y = HEX_GQ * hex_sign(g, 1), z = HEX_GQ * hex_sign(g, 2);
-      double J[9], iJ[9], G[9], H[9];
-      hex_modal_grad(cm, x, y, z, J);
-      const double detJ = inv3(J, iJ);
-      hex_modal_grad(um, x, y, z, G);
-      matmul3(G, iJ, H);
-      const double bb = (tr0 - (H[0] + H[4] + H[8])) / 3.0;
-      H[0] += bb;
-      H[4] += bb;
-      H[8] += bb;
-      double sig[6], tn[8];
-      const double* st = st_e ? st_e + g * ns : zero_state;
-      material_stress(mat, lam_k, mu_k, H, st, sn_e ? sn_e + g * ns : nullptr, sig, tn);
-      if (MODE != FORCE_STRESS) {
-        if (tan64)
-#pragma unroll
-          for (int k = 0; k < 8; ++k) tan64[tile_index(tpos[e], g * 8 + k, NG * 8, tile)] = tn[k];
-        if (tan32)
-#pragma unroll
-          for (int k = 0; k < 8; ++k) tan32[tile_index(tpos[e], g * 8 + k, NG * 8, tile)] = (float)tn[k];
-      }
-      if (MODE == FORCE_FULL) {
-        const double vol = detJ * sc;
-        const double t = vol * (sig[0] + sig[1] + sig[2]) / 3.0;
-        tacc += t;
-        double cdev[6] = {vol * sig[0] - t, vol * sig[1] - t, vol * sig[2] - t,
-                          vol * sig[3], vol * sig[4], vol * sig[5]};
-        double Q[9];
-        cotangent(cdev, 1.0, iJ, Q);
-        hex_modal_grad_adj(Q, x, y, z, Fm);
-      } else if (MODE == FORCE_STRESS) {
-        double snew[19];
-        material_stress(mat, lam_k, mu_k, H, st, snew, sig, tn);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) Sacc[k] += detJ * sig[k];
-        vsum += detJ;
-        if (mat.kind == EXFEM_J2) pacc += detJ * snew[9];
-      }
-    }
-    if (MODE == FORCE_FULL && fe) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int i = 0; i < 3; ++i) Fm[i][c] += tacc * iJ0[3 * i + c];
-      double f[8][3];
-      hex_from_modal(Fm, f);
-#pragma unroll
-      for (int a = 0; a < 8; ++a)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) fe[(e * 8 + a) * 3 + c] = f[a][c];
-    }
-  } else {
-    double f[10][3];
-#pragma unroll
-    for (int a = 0; a < 10; ++a) f[a][0] = f[a][1] = f[a][2] = 0.0;
-#pragma unroll 1
-    for (int g = 0; g < 4; ++g) {
-      double J[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, iJ[9], H[9];
-#pragma unroll
-      for (int a = 0; a < 10; ++a) {
-        const int64_t n3 = 3 * (int64_t)nod[a];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          double dn = 0.0;
-          // compile-time table lookup (g is a runtime loop index)
-          switch (g) {
-            case 0: dn = tet10_dN(0, a, i); break;
-            case 1: dn = tet10_dN(1, a, i); break;
-            case 2: dn = tet10_dN(2, a, i); break;
-            default: dn = tet10_dN(3, a, i); break;
-          }
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            J[3 * c + i] += X[n3 + c] * dn;
-            G[3 * c + i] += u[n3 + c] * dn;
-          }
-        }
-      }
-      const double detJ = inv3(J, iJ);
-      matmul3(G, iJ, H);
-      double sig[6], tn[8];
-      const double* st = st_e ? st_e + g * ns : zero_state;
-      material_stress(mat, lam_k, mu_k, H, st, sn_e ? sn_e + g * ns : nullptr, sig, tn);
-      if (MODE != FORCE_STRESS) {
-        if (tan64)
-#pragma unroll
-          for (int k = 0; k < 8; ++k) tan64[tile_index(tpos[e], g * 8 + k, NG * 8, tile)] = tn[k];
-        if (tan32)
-#pragma unroll
-          for (int k = 0; k < 8; ++k) tan32[tile_index(tpos[e], g * 8 + k, NG * 8, tile)] = (float)tn[k];
-      }
-      if (MODE == FORCE_FULL) {
-        const double vol = detJ / 24.0 * sc;
-        double Q[9];
-        cotangent(sig, vol, iJ, Q);
-#pragma unroll
-        for (int a = 0; a < 10; ++a)
-#pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            double dn = 0.0;
-            switch (g) {
-              case 0: dn = tet10_dN(0, a, i); break;
-              case 1: dn = tet10_dN(1, a, i); break;
-              case 2: dn = tet10_dN(2, a, i); break;
-              default: dn = tet10_dN(3, a, i); break;
-            }
-#pragma unroll
-            for (int c = 0; c < 3; ++c) f[a][c] += Q[3 * c + i] * dn;
-          }
-      } else if (MODE == FORCE_STRESS) {
-        double snew[19];
-        material_stress(mat, lam_k, mu_k, H, st, snew, sig, tn);
-        const double w = detJ / 24.0;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) Sacc[k] += w * sig[k];
-        vsum += w;
-        if (mat.kind == EXFEM_J2) pacc += w * snew[9];
-      }
-    }
-    if (MODE == FORCE_FULL && fe) {
-#pragma unroll
-      for (int a = 0; a < 10; ++a)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) fe[(e * 10 + a) * 3 + c] = f[a][c];
-    }
-  }
-  if (MODE == FORCE_STRESS) {
-    double s[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) s[k] = Sacc[k] / vsum;
-    if (S) {
-      double* o = S + e * 9;
-      o[0] = s[0]; o[1] = s[3]; o[2] = s[5];
-      o[3] = s[3]; o[4] = s[1]; o[5] = s[4];
-      o[6] = s[5]; o[7] = s[4]; o[8] = s[2];
-    }
-    const double m3 = (s[0] + s[1] + s[2]) / 3.0;
-    const double d0 = s[0] - m3, d1 = s[1] - m3, d2 = s[2] - m3;
-    if (mises)
-      mises[e] = sqrt(1.5 * (d0 * d0 + d1 * d1 + d2 * d2 + 2.0 * (s[3] * s[3] + s[4] * s[4] + s[5] * s[5])));
-    if (peeq) peeq[e] = pacc / vsum;
-  }
-}
-
-template <int ET, int MODE>
-static int force_dispatch(exfem_block_s* b, const double* u, const double* st_old, double* st_new,
-                          double* fe, double* S, double* mises, double* peeq, cudaStream_t s) {
-  const int threads = 128;
-  const unsigned grid = (unsigned)((b->ne + threads - 1) / threads);
-  const bool j2 = b->mat.kind == EXFEM_J2;
-  double* t64 = (MODE != FORCE_STRESS && j2) ? b->tan64.p : nullptr;
-  float* t32 = (MODE != FORCE_STRESS && j2) ? b->tan32.p : nullptr;
-  force_kernel<ET, MODE><<<grid, threads, 0, s>>>(b->ne, b->X.p, b->conn.p, u, b->scale.p, st_old,
-                                                  st_new, fe, t64, t32, S, mises, peeq, b->mat, b->lam_e.p,
-                                                  b->mu_e.p, b->tpos.p, b->tile);
-  EX_LAUNCH_CHECK();
-  return EXFEM_OK;
-}
-
-int launch_force(exfem_block_s* b, int mode, const double* u, const double* st_old, double* st_new,
-                 double* fe, double* S, double* mises, double* peeq, cudaStream_t s) {
-  if (b->ne == 0) return EXFEM_OK;
-#define EXF_CASE(ET)                                                                           \
-  if (b->etype == ET) {                                                                        \
-    if (mode == FORCE_FULL) return force_dispatch<ET, FORCE_FULL>(b, u, st_old, st_new, fe, S, mises, peeq, s); \
-    if (mode == FORCE_TANGENT) return force_dispatch<ET, FORCE_TANGENT>(b, u, st_old, st_new, fe, S, mises, peeq, s); \
-    return force_dispatch<ET, FORCE_STRESS>(b, u, st_old, st_new, fe, S, mises, peeq, s);      \
-  }
-  EXF_CASE(EXFEM_C3D8)
-  EXF_CASE(EXFEM_C3D10)
-#undef EXF_CASE
-  set_error("unknown element type %d", b->etype);
-  return EXFEM_ERR_ARG;
-}
 
 // ---------------------------------------------------------------- assembly
 // f[3n+c] = sum over the gather plan of node n (reference order); optional opA

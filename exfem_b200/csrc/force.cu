@@ -1,0 +1,345 @@
+// FP64 internal force with the J2 return map and the consistent-tangent data it
+// produces, the tangent data alone, and element-averaged stresses
+// (gfem/model.py:35-81, 129-137, 466-486).
+//
+// One warp takes 32 / ngp elements (4 C3D8, 8 C3D10), one lane per Gauss point.  Node
+// values are gathered once per element and Gauss-point states in whole lines into the
+// warp's shared memory; a lane evaluates its point's kinematics and material; the
+// element forces
+//   f_a = sum_g sum_i dN_a/dxi_i(g) Q_g[:, i],  Q_g = vol sigma J^-T,
+// are one small product of the constant dN table with the Q of all the warp's elements
+// side by side, done with the FP64 matrix instruction, which also sums over the lanes;
+// under B-bar (C3D8) the mean stress acts through the gradients at the centre, three
+// more rows of the same product.  New states and forces leave in whole lines.
+//
+// J2 blocks are walked in tile order, in which the tangent data of neighbouring
+// elements are neighbours in memory; otherwise elements are taken as they are numbered.
+//
+// Measured on B200, with the assembly: 40,000 J2 C3D8 63 us, 125,550 J2 C3D10 104 us
+// (states read and written, tangent data written); one thread per element, which read
+// each state entry with a stride of a whole element, took 170 and 212 us.  Bound by
+// instruction issue and the shared-memory pipe (0.40 and 0.68 busy) at 16 warps an SM.
+#include "async_copy.cuh"
+#include "internal.h"
+
+namespace exfem {
+
+namespace {
+
+// dN_b / dxi_i at every Gauss point, rows of 3 nnode + 1: the odd stride puts the
+// points' rows into different banks
+template <int ET>
+struct DnTable {
+  static constexpr int NN = ElemTraits<ET>::nnode, NG = ElemTraits<ET>::ngp, XS = 3 * NN + 1;
+  double v[NG * XS];
+  constexpr DnTable() : v{} {
+    for (int g = 0; g < NG; ++g)
+      for (int b = 0; b < NN; ++b)
+        for (int i = 0; i < 3; ++i) v[g * XS + 3 * b + i] = ET == EXFEM_C3D8 ? hex_dN(g, b, i) : tet10_dN(g, b, i);
+  }
+};
+__device__ const DnTable<EXFEM_C3D8> dn_hex{};
+__device__ const DnTable<EXFEM_C3D10> dn_tet{};
+template <int ET>
+__device__ __forceinline__ const double* dn_table() {
+  if constexpr (ET == EXFEM_C3D8) return dn_hex.v;
+  else return dn_tet.v;
+}
+
+// shared memory of one warp
+template <int ET, bool J2>
+struct ForceSmem {
+  using Tr = ElemTraits<ET>;
+  static constexpr int NN = Tr::nnode, NG = Tr::ngp, ND = 3 * NN, EPW = 32 / NG, XS = 3 * NN + 1;
+  static constexpr bool BBAR = ET == EXFEM_C3D8;
+  union {  // node values, then Q of every Gauss point, then element forces
+    struct {
+      double x[EPW * XS], u[EPW * XS];
+    };
+    double Q[9][33];  // odd stride for the gathers below
+    double F[EPW * ND];
+  };
+  double c0[BBAR ? EPW : 1][19];  // J and du/dxi at the centre; then mean stress times J0^-1
+  double st[J2 ? 32 * 19 : 1];    // Gauss-point states: the lanes' stride of 19 meets no bank conflict
+};
+
+template <int ET, bool J2, int MODE, int NW>
+__global__ void __launch_bounds__(32 * NW, 16 / NW)
+force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict__ conn,
+             const double* __restrict__ u, const double* __restrict__ scale, const double* st_old, double* st_new,
+             double* __restrict__ fe, double* __restrict__ tan64, float* __restrict__ tan32, double* __restrict__ S,
+             double* __restrict__ mises, double* __restrict__ peeq, const __grid_constant__ MatDev mat,
+             const double* __restrict__ lam_e, const double* __restrict__ mu_e, const int32_t* __restrict__ order,
+             int tile) {
+  using SM = ForceSmem<ET, J2>;
+  constexpr int NN = SM::NN, NG = SM::NG, ND = SM::ND, EPW = SM::EPW, XS = SM::XS;
+  constexpr bool BBAR = SM::BBAR;
+  constexpr bool TILED = J2 && MODE != FORCE_STRESS;  // walked in tile order
+  constexpr int MT = NN > 8 ? 2 : 1, NTC = (3 * EPW + 7) / 8, KS = NG * 3 / 4 + (BBAR ? 1 : 0);
+  __shared__ double tab[NG * XS];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  SM& sm = reinterpret_cast<SM*>(smem_raw)[warp];
+  for (int k = threadIdx.x; k < NG * XS; k += 32 * NW) tab[k] = dn_table<ET>()[k];
+  __syncthreads();
+  const int64_t p0 = ((int64_t)blockIdx.x * NW + warp) * EPW;
+  if (p0 >= ne) return;
+  const int cnt = ne - p0 < EPW ? (int)(ne - p0) : EPW;
+  const int le = lane / NG, g = lane % NG;
+  const bool valid = le < cnt;
+  const int64_t pos = p0 + (valid ? le : 0);
+  const int32_t eid = TILED ? order[pos] : (int32_t)pos;  // this lane's element
+  // element of the warp's el-th position, on every lane
+  auto elem = [&](int el) { return TILED ? (int64_t)__shfl_sync(0xffffffffu, eid, el * NG) : p0 + el; };
+
+  // ---- states and node values of the warp's elements
+  if (J2 && st_old) {
+#pragma unroll
+    for (int k0 = 0; k0 < 32 * 19; k0 += 32) {
+      const int k = k0 + lane, el = k / (NG * 19);
+      const int64_t e = elem(el);
+      if (el < cnt) cp_async<8>(sm.st + k, st_old + e * (NG * 19) + (k - el * (NG * 19)), 8);
+    }
+  }
+#pragma unroll
+  for (int k0 = 0; k0 < EPW * NN; k0 += 32) {
+    const int k = k0 + lane, el = k / NN < EPW ? k / NN : EPW - 1;
+    const int64_t e = elem(el);
+    if (k < cnt * NN) {
+      const int a = k - el * NN;
+      const int64_t n3 = 3 * (int64_t)conn[e * NN + a];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        sm.x[el * XS + 3 * a + c] = X[n3 + c];
+        sm.u[el * XS + 3 * a + c] = u[n3 + c];
+      }
+    }
+  }
+  if constexpr (J2) cp_async_wait_all();
+  __syncwarp();
+  if constexpr (BBAR) {  // gradients at the centre: 18 sums an element, spread over its lanes
+    const double* xe = sm.x + le * XS;
+    for (int k = g; k < 18; k += NG) {
+      const int o = k >= 9 ? EPW * XS : 0, c = (k % 9) / 3, i = k % 3;  // u follows x
+      double s = 0.0;
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        const double v = xe[o + 3 * b + c];
+        s += hex_sign(b, i) > 0 ? v : -v;
+      }
+      sm.c0[le][k] = 0.125 * s;
+    }
+    __syncwarp();
+  }
+
+  // ---- this lane's Gauss point
+  const double lam_k = lam_e ? lam_e[eid] : mat.lam, mu_k = lam_e ? mu_e[eid] : mat.mu;
+  double J[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, iJ[9], iJ0[9], H[9];
+  {
+    const double* dn = tab + g * XS;
+    const double *xe = sm.x + le * XS, *ue = sm.u + le * XS;
+#pragma unroll
+    for (int b = 0; b < NN; ++b)
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          J[3 * c + i] += xe[3 * b + c] * dn[3 * b + i];
+          G[3 * c + i] += ue[3 * b + c] * dn[3 * b + i];
+        }
+  }
+  const double detJ = inv3(J, iJ);
+  matmul3(G, iJ, H);
+  if constexpr (BBAR) {
+    double J0[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) J0[k] = sm.c0[le][k];
+    inv3(J0, iJ0);
+    double tr0 = 0.0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int i = 0; i < 3; ++i) tr0 += sm.c0[le][9 + 3 * c + i] * iJ0[3 * i + c];
+    const double bb = (tr0 - (H[0] + H[4] + H[8])) * (1.0 / 3.0);
+    H[0] += bb;
+    H[4] += bb;
+    H[8] += bb;
+  }
+  double sig[6], tn[8], alpha = 0.0;
+  if constexpr (J2) {
+    double* st = sm.st + lane * 19;
+    if (!st_old)
+#pragma unroll
+      for (int k = 0; k < 19; ++k) st[k] = 0.0;
+    double e[6], sn[19];
+    sym_from_grad(H, e);
+    j2_return(mat, e, st, MODE == FORCE_TANGENT ? nullptr : sn, sig, tn);
+    alpha = sn[9];
+    if (MODE == FORCE_FULL)
+#pragma unroll
+      for (int k = 0; k < 19; ++k) st[k] = sn[k];
+  } else {
+    double e[6];
+    sym_from_grad(H, e);
+    elastic_stress(lam_k, mu_k, e, sig);
+    if (MODE == FORCE_FULL && st_new && valid)
+      st_new[(int64_t)eid * NG + g] = st_old ? st_old[(int64_t)eid * NG + g] : 0.0;
+  }
+  const double vol = (BBAR ? 1.0 : 1.0 / 24.0) * detJ * (MODE != FORCE_STRESS && scale ? scale[eid] : 1.0);
+
+  if constexpr (TILED) {
+    if (valid) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int64_t o = tile_index(pos, g * 8 + k, NG * 8, tile);
+        tan64[o] = tn[k];
+        tan32[o] = (float)tn[k];
+      }
+    }
+  }
+
+  if constexpr (MODE == FORCE_STRESS) {
+    // volume averages over the element's lanes
+    double a[8];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) a[k] = vol * sig[k];
+    a[6] = vol;
+    a[7] = vol * alpha;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+#pragma unroll
+      for (int o = NG / 2; o > 0; o >>= 1) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
+    if (valid && g == 0) {
+      double s[6];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) s[k] = a[k] / a[6];
+      if (S) {
+        double* o = S + (int64_t)eid * 9;
+        o[0] = s[0]; o[1] = s[3]; o[2] = s[5];
+        o[3] = s[3]; o[4] = s[1]; o[5] = s[4];
+        o[6] = s[5]; o[7] = s[4]; o[8] = s[2];
+      }
+      const double m3 = (s[0] + s[1] + s[2]) / 3.0;
+      const double d0 = s[0] - m3, d1 = s[1] - m3, d2 = s[2] - m3;
+      if (mises)
+        mises[eid] = sqrt(1.5 * (d0 * d0 + d1 * d1 + d2 * d2 + 2.0 * (s[3] * s[3] + s[4] * s[4] + s[5] * s[5])));
+      if (peeq) peeq[eid] = J2 ? a[7] / a[6] : 0.0 / a[6];
+    }
+  }
+
+  if constexpr (MODE == FORCE_FULL) {
+    // Q = vol sigma J^-T; under B-bar the deviatoric part, and the mean stress of the
+    // element times the gradients at its centre
+    double t = 0.0;
+    if constexpr (BBAR) {
+      t = vol * (sig[0] + sig[1] + sig[2]) * (1.0 / 3.0);
+      double tacc = t;
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) tacc += __shfl_xor_sync(0xffffffffu, tacc, o);
+      if (g == 0)  // the centre's values were read before the shuffles above
+#pragma unroll
+        for (int k = 0; k < 9; ++k) sm.c0[le][k] = tacc * iJ0[k];
+    }
+    const double r[3][3] = {{vol * sig[0] - t, vol * sig[3], vol * sig[5]},
+                            {vol * sig[3], vol * sig[1] - t, vol * sig[4]},
+                            {vol * sig[5], vol * sig[4], vol * sig[2] - t}};
+    __syncwarp();  // node values read by every lane; new states in place
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        sm.Q[3 * c + i][lane] = r[c][0] * iJ[3 * i] + r[c][1] * iJ[3 * i + 1] + r[c][2] * iJ[3 * i + 2];
+    if (J2 && st_new) {
+#pragma unroll
+      for (int k0 = 0; k0 < 32 * 19; k0 += 32) {
+        const int k = k0 + lane, el = k / (NG * 19);
+        const int64_t e = elem(el);
+        if (el < cnt) st_new[e * (NG * 19) + (k - el * (NG * 19))] = sm.st[k];
+      }
+    }
+    __syncwarp();
+    const int row = lane >> 2, q = lane & 3;
+    double f[MT][NTC][2];
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int n = 0; n < NTC; ++n) f[m][n][0] = f[m][n][1] = 0.0;
+#pragma unroll
+    for (int s = 0; s < KS; ++s) {
+      const bool centre = BBAR && s == KS - 1;  // k: the three rows of the centre, one empty
+      const int kk = 4 * s + q, gk = kk / 3, i = centre ? q : kk % 3;
+      double a[MT], b[NTC];
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        const int node = 8 * m + row;
+        if (centre) a[m] = q < 3 ? 0.125 * hex_sign(node & 7, q) : 0.0;
+        else a[m] = node < NN ? tab[gk * XS + 3 * node + i] : 0.0;
+      }
+#pragma unroll
+      for (int n = 0; n < NTC; ++n) {
+        const int col = 8 * n + row, el = col / 3, c = col % 3;
+        if (centre) b[n] = q < 3 && el < EPW ? sm.c0[el < EPW ? el : 0][3 * i + c] : 0.0;
+        else b[n] = el < EPW ? sm.Q[3 * c + i][el * NG + gk] : 0.0;
+      }
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int n = 0; n < NTC; ++n) dmma(f[m][n], a[m], b[n]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int n = 0; n < NTC; ++n)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int node = 8 * m + row, col = 8 * n + 2 * q + h;
+          if (node < NN && col < 3 * EPW) sm.F[(col / 3) * ND + 3 * node + col % 3] = f[m][n][h];
+        }
+    __syncwarp();
+#pragma unroll
+    for (int k0 = 0; k0 < EPW * ND; k0 += 32) {
+      const int k = k0 + lane, el = k / ND < EPW ? k / ND : EPW - 1;
+      const int64_t e = elem(el);
+      if (k < cnt * ND) fe[e * ND + (k - el * ND)] = sm.F[k];
+    }
+  }
+}
+
+template <int ET, bool J2, int MODE>
+int force_go(exfem_block_s* b, const double* u, const double* st_old, double* st_new, double* fe, double* S,
+             double* mises, double* peeq, cudaStream_t s) {
+  constexpr int NW = 4;
+  using SM = ForceSmem<ET, J2>;
+  constexpr size_t smem = NW * sizeof(SM);
+  constexpr int64_t per = NW * SM::EPW;
+  force_kernel<ET, J2, MODE, NW><<<(unsigned)((b->ne + per - 1) / per), 32 * NW, smem, s>>>(
+      b->ne, b->X.p, b->conn.p, u, b->scale.p, st_old, st_new, fe, b->tan64.p, b->tan32.p, S, mises, peeq, b->mat,
+      b->lam_e.p, b->mu_e.p, b->order_dev.p, b->tile);
+  EX_LAUNCH_CHECK();
+  return EXFEM_OK;
+}
+
+template <int ET>
+int force_et(exfem_block_s* b, int mode, const double* u, const double* st_old, double* st_new, double* fe, double* S,
+             double* mises, double* peeq, cudaStream_t s) {
+  if (b->mat.kind == EXFEM_J2) {
+    if (mode == FORCE_FULL) return force_go<ET, true, FORCE_FULL>(b, u, st_old, st_new, fe, S, mises, peeq, s);
+    if (mode == FORCE_TANGENT) return force_go<ET, true, FORCE_TANGENT>(b, u, st_old, st_new, fe, S, mises, peeq, s);
+    return force_go<ET, true, FORCE_STRESS>(b, u, st_old, st_new, fe, S, mises, peeq, s);
+  }
+  if (mode == FORCE_FULL) return force_go<ET, false, FORCE_FULL>(b, u, st_old, st_new, fe, S, mises, peeq, s);
+  if (mode == FORCE_TANGENT) return EXFEM_OK;  // an elastic tangent does not change
+  return force_go<ET, false, FORCE_STRESS>(b, u, st_old, st_new, fe, S, mises, peeq, s);
+}
+
+}  // namespace
+
+int launch_force(exfem_block_s* b, int mode, const double* u, const double* st_old, double* st_new, double* fe,
+                 double* S, double* mises, double* peeq, cudaStream_t s) {
+  if (b->ne == 0) return EXFEM_OK;
+  return b->etype == EXFEM_C3D8 ? force_et<EXFEM_C3D8>(b, mode, u, st_old, st_new, fe, S, mises, peeq, s)
+                                : force_et<EXFEM_C3D10>(b, mode, u, st_old, st_new, fe, S, mises, peeq, s);
+}
+
+}  // namespace exfem
