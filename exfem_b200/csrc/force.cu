@@ -15,52 +15,33 @@
 // J2 blocks are walked in tile order, in which the tangent data of neighbouring
 // elements are neighbours in memory; otherwise elements are taken as they are numbered.
 //
-// Measured on B200, with the assembly: 40,000 J2 C3D8 63 us, 125,550 J2 C3D10 104 us
+// Measured on B200, with the assembly: 40,000 J2 C3D8 51 us, 125,550 J2 C3D10 89 us
 // (states read and written, tangent data written); one thread per element, which read
-// each state entry with a stride of a whole element, took 170 and 212 us.  Bound by
-// instruction issue and the shared-memory pipe (0.40 and 0.68 busy) at 16 warps an SM.
-#include "async_copy.cuh"
+// each state entry with a stride of a whole element, took 170 and 212 us, and copying
+// states entry by entry instead of in bulk 63 and 104 us.
+#include "gauss_warp.cuh"
 #include "internal.h"
 
 namespace exfem {
 
 namespace {
 
-// dN_b / dxi_i at every Gauss point, rows of 3 nnode + 1: the odd stride puts the
-// points' rows into different banks
-template <int ET>
-struct DnTable {
-  static constexpr int NN = ElemTraits<ET>::nnode, NG = ElemTraits<ET>::ngp, XS = 3 * NN + 1;
-  double v[NG * XS];
-  constexpr DnTable() : v{} {
-    for (int g = 0; g < NG; ++g)
-      for (int b = 0; b < NN; ++b)
-        for (int i = 0; i < 3; ++i) v[g * XS + 3 * b + i] = ET == EXFEM_C3D8 ? hex_dN(g, b, i) : tet10_dN(g, b, i);
-  }
-};
-__device__ const DnTable<EXFEM_C3D8> dn_hex{};
-__device__ const DnTable<EXFEM_C3D10> dn_tet{};
-template <int ET>
-__device__ __forceinline__ const double* dn_table() {
-  if constexpr (ET == EXFEM_C3D8) return dn_hex.v;
-  else return dn_tet.v;
-}
+enum BulkArrays { BULK_OLD = 1, BULK_NEW = 2, BULK_FE = 4 };
 
 // shared memory of one warp
 template <int ET, bool J2>
 struct ForceSmem {
   using Tr = ElemTraits<ET>;
-  static constexpr int NN = Tr::nnode, NG = Tr::ngp, ND = 3 * NN, EPW = 32 / NG, XS = 3 * NN + 1;
+  static constexpr int NN = Tr::nnode, NG = Tr::ngp, ND = 3 * NN, EPW = 32 / NG, ST = NG * 19;
   static constexpr bool BBAR = ET == EXFEM_C3D8;
-  union {  // node values, then Q of every Gauss point, then element forces
-    struct {
-      double x[EPW * XS], u[EPW * XS];
-    };
-    double Q[9][33];  // odd stride for the gathers below
-    double F[EPW * ND];
+  alignas(16) double st[J2 ? 32 * 19 : 2];  // Gauss-point states: the lanes' stride of 19 meets no bank conflict
+  union {                                   // node values, then Q of every Gauss point, then element forces
+    NodeSmem<ET, true> nd;
+    double Q[9][33];  // odd stride for the gathers of the matrix product
+    alignas(16) double F[EPW * ND];
   };
-  double c0[BBAR ? EPW : 1][19];  // J and du/dxi at the centre; then mean stress times J0^-1
-  double st[J2 ? 32 * 19 : 1];    // Gauss-point states: the lanes' stride of 19 meets no bank conflict
+  double c0[BBAR ? EPW : 1][9];  // mean stress times the inverse Jacobian of the centre
+  uint64_t bar;                  // arrival of the states
 };
 
 template <int ET, bool J2, int MODE, int NW>
@@ -70,13 +51,13 @@ force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict
              double* __restrict__ fe, double* __restrict__ tan64, float* __restrict__ tan32, double* __restrict__ S,
              double* __restrict__ mises, double* __restrict__ peeq, const __grid_constant__ MatDev mat,
              const double* __restrict__ lam_e, const double* __restrict__ mu_e, const int32_t* __restrict__ order,
-             int tile) {
+             int tile_log2, int bulk, int* __restrict__ err) {
   using SM = ForceSmem<ET, J2>;
-  constexpr int NN = SM::NN, NG = SM::NG, ND = SM::ND, EPW = SM::EPW, XS = SM::XS;
+  constexpr int NN = SM::NN, NG = SM::NG, ND = SM::ND, EPW = SM::EPW, ST = SM::ST, XS = DnTable<ET>::XS;
   constexpr bool BBAR = SM::BBAR;
   constexpr bool TILED = J2 && MODE != FORCE_STRESS;  // walked in tile order
   constexpr int MT = NN > 8 ? 2 : 1, NTC = (3 * EPW + 7) / 8, KS = NG * 3 / 4 + (BBAR ? 1 : 0);
-  __shared__ double tab[NG * XS];
+  __shared__ __align__(16) double tab[NG * XS];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   SM& sm = reinterpret_cast<SM*>(smem_raw)[warp];
@@ -92,74 +73,41 @@ force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict
   // element of the warp's el-th position, on every lane
   auto elem = [&](int el) { return TILED ? (int64_t)__shfl_sync(0xffffffffu, eid, el * NG) : p0 + el; };
 
-  // ---- states and node values of the warp's elements
+  // ---- states (whole elements, one bulk copy each) and node values
   if (J2 && st_old) {
-#pragma unroll
-    for (int k0 = 0; k0 < 32 * 19; k0 += 32) {
-      const int k = k0 + lane, el = k / (NG * 19);
-      const int64_t e = elem(el);
-      if (el < cnt) cp_async<8>(sm.st + k, st_old + e * (NG * 19) + (k - el * (NG * 19)), 8);
-    }
-  }
-#pragma unroll
-  for (int k0 = 0; k0 < EPW * NN; k0 += 32) {
-    const int k = k0 + lane, el = k / NN < EPW ? k / NN : EPW - 1;
-    const int64_t e = elem(el);
-    if (k < cnt * NN) {
-      const int a = k - el * NN;
-      const int64_t n3 = 3 * (int64_t)conn[e * NN + a];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        sm.x[el * XS + 3 * a + c] = X[n3 + c];
-        sm.u[el * XS + 3 * a + c] = u[n3 + c];
+    if (bulk & BULK_OLD) {
+      if (lane == 0) {
+        mbar_init(&sm.bar, 1);
+        fence_mbar_init();
+        mbar_expect_tx(&sm.bar, cnt * ST * (uint32_t)sizeof(double));
+      }
+      __syncwarp();
+      if (valid && g == 0)
+        bulk_g2s(sm.st + le * ST, st_old + (int64_t)eid * ST, ST * (uint32_t)sizeof(double), &sm.bar);
+    } else {
+      for (int k0 = 0; k0 < 32 * 19; k0 += 32) {
+        const int k = k0 + lane, el = k / ST;
+        const int64_t e = elem(el);
+        if (el < cnt) cp_async<8>(sm.st + k, st_old + e * ST + (k - el * ST), 8);
       }
     }
   }
-  if constexpr (J2) cp_async_wait_all();
+  gather_nodes<ET, true>(sm.nd, X, conn, u, eid, cnt, elem);
   __syncwarp();
-  if constexpr (BBAR) {  // gradients at the centre: 18 sums an element, spread over its lanes
-    const double* xe = sm.x + le * XS;
-    for (int k = g; k < 18; k += NG) {
-      const int o = k >= 9 ? EPW * XS : 0, c = (k % 9) / 3, i = k % 3;  // u follows x
-      double s = 0.0;
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        const double v = xe[o + 3 * b + c];
-        s += hex_sign(b, i) > 0 ? v : -v;
-      }
-      sm.c0[le][k] = 0.125 * s;
-    }
-    __syncwarp();
-  }
 
   // ---- this lane's Gauss point
   const double lam_k = lam_e ? lam_e[eid] : mat.lam, mu_k = lam_e ? mu_e[eid] : mat.mu;
-  double J[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, iJ[9], iJ0[9], H[9];
-  {
-    const double* dn = tab + g * XS;
-    const double *xe = sm.x + le * XS, *ue = sm.u + le * XS;
-#pragma unroll
-    for (int b = 0; b < NN; ++b)
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          J[3 * c + i] += xe[3 * b + c] * dn[3 * b + i];
-          G[3 * c + i] += ue[3 * b + c] * dn[3 * b + i];
-        }
-  }
+  double J[9], G[9], J0[9], G0[9], iJ[9], iJ0[9], H[9];
+  gauss_gradients<ET, true>(sm.nd, tab, le, g, J, G, J0, G0);
   const double detJ = inv3(J, iJ);
   matmul3(G, iJ, H);
   if constexpr (BBAR) {
-    double J0[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) J0[k] = sm.c0[le][k];
     inv3(J0, iJ0);
     double tr0 = 0.0;
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
-      for (int i = 0; i < 3; ++i) tr0 += sm.c0[le][9 + 3 * c + i] * iJ0[3 * i + c];
+      for (int i = 0; i < 3; ++i) tr0 += G0[3 * c + i] * iJ0[3 * i + c];
     const double bb = (tr0 - (H[0] + H[4] + H[8])) * (1.0 / 3.0);
     H[0] += bb;
     H[4] += bb;
@@ -168,9 +116,15 @@ force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict
   double sig[6], tn[8], alpha = 0.0;
   if constexpr (J2) {
     double* st = sm.st + lane * 19;
-    if (!st_old)
+    if (!st_old) {
 #pragma unroll
       for (int k = 0; k < 19; ++k) st[k] = 0.0;
+    } else if (bulk & BULK_OLD) {
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(&sm.bar, 0, err))) return;
+    } else {
+      cp_async_wait_all();
+      __syncwarp();
+    }
     double e[6], sn[19];
     sym_from_grad(H, e);
     j2_return(mat, e, st, MODE == FORCE_TANGENT ? nullptr : sn, sig, tn);
@@ -189,9 +143,11 @@ force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict
 
   if constexpr (TILED) {
     if (valid) {
+      // tile_index(pos, 8 g + k, 8 ngp, tile) for a power of two
+      const int64_t o0 = (((pos >> tile_log2) * (NG * 8) + g * 8) << tile_log2) + (pos & ((1 << tile_log2) - 1));
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const int64_t o = tile_index(pos, g * 8 + k, NG * 8, tile);
+        const int64_t o = o0 + (k << tile_log2);
         tan64[o] = tn[k];
         tan32[o] = (float)tn[k];
       }
@@ -236,7 +192,7 @@ force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict
       double tacc = t;
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1) tacc += __shfl_xor_sync(0xffffffffu, tacc, o);
-      if (g == 0)  // the centre's values were read before the shuffles above
+      if (g == 0)
 #pragma unroll
         for (int k = 0; k < 9; ++k) sm.c0[le][k] = tacc * iJ0[k];
     }
@@ -250,11 +206,19 @@ force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict
       for (int i = 0; i < 3; ++i)
         sm.Q[3 * c + i][lane] = r[c][0] * iJ[3 * i] + r[c][1] * iJ[3 * i + 1] + r[c][2] * iJ[3 * i + 2];
     if (J2 && st_new) {
-#pragma unroll
-      for (int k0 = 0; k0 < 32 * 19; k0 += 32) {
-        const int k = k0 + lane, el = k / (NG * 19);
-        const int64_t e = elem(el);
-        if (el < cnt) st_new[e * (NG * 19) + (k - el * (NG * 19))] = sm.st[k];
+      if (bulk & BULK_NEW) {
+        fence_proxy_async();
+        __syncwarp();
+        if (valid && g == 0) {
+          bulk_s2g(st_new + (int64_t)eid * ST, sm.st + le * ST, ST * (uint32_t)sizeof(double));
+          bulk_commit();
+        }
+      } else {
+        for (int k0 = 0; k0 < 32 * 19; k0 += 32) {
+          const int k = k0 + lane, el = k / ST;
+          const int64_t e = elem(el);
+          if (el < cnt) st_new[e * ST + (k - el * ST)] = sm.st[k];
+        }
       }
     }
     __syncwarp();
@@ -296,13 +260,22 @@ force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict
           const int node = 8 * m + row, col = 8 * n + 2 * q + h;
           if (node < NN && col < 3 * EPW) sm.F[(col / 3) * ND + 3 * node + col % 3] = f[m][n][h];
         }
-    __syncwarp();
-#pragma unroll
-    for (int k0 = 0; k0 < EPW * ND; k0 += 32) {
-      const int k = k0 + lane, el = k / ND < EPW ? k / ND : EPW - 1;
-      const int64_t e = elem(el);
-      if (k < cnt * ND) fe[e * ND + (k - el * ND)] = sm.F[k];
+    if (bulk & BULK_FE) {
+      fence_proxy_async();
+      __syncwarp();
+      if (valid && g == 0) {
+        bulk_s2g(fe + (int64_t)eid * ND, sm.F + le * ND, ND * (uint32_t)sizeof(double));
+        bulk_commit();
+      }
+    } else {
+      __syncwarp();
+      for (int k0 = 0; k0 < EPW * ND; k0 += 32) {
+        const int k = k0 + lane, el = k / ND < EPW ? k / ND : EPW - 1;
+        const int64_t e = elem(el);
+        if (k < cnt * ND) fe[e * ND + (k - el * ND)] = sm.F[k];
+      }
     }
+    bulk_wait_read<0>();  // shared memory stays until the copies have read it
   }
 }
 
@@ -313,9 +286,13 @@ int force_go(exfem_block_s* b, const double* u, const double* st_old, double* st
   using SM = ForceSmem<ET, J2>;
   constexpr size_t smem = NW * sizeof(SM);
   constexpr int64_t per = NW * SM::EPW;
+  // bulk copies need 16-byte boundaries: elements' states and forces are multiples of
+  // 16 bytes, so it takes the arrays themselves to start on one
+  const int bulk = ((uintptr_t)st_old % 16 == 0 ? BULK_OLD : 0) | ((uintptr_t)st_new % 16 == 0 ? BULK_NEW : 0) |
+                   ((uintptr_t)fe % 16 == 0 ? BULK_FE : 0);
   force_kernel<ET, J2, MODE, NW><<<(unsigned)((b->ne + per - 1) / per), 32 * NW, smem, s>>>(
       b->ne, b->X.p, b->conn.p, u, b->scale.p, st_old, st_new, fe, b->tan64.p, b->tan32.p, S, mises, peeq, b->mat,
-      b->lam_e.p, b->mu_e.p, b->order_dev.p, b->tile);
+      b->lam_e.p, b->mu_e.p, b->order_dev.p, b->tile == 128 ? 7 : 8, bulk, b->dev_err.p);
   EX_LAUNCH_CHECK();
   return EXFEM_OK;
 }

@@ -19,7 +19,7 @@
 // of three rows of Ke.
 #include <cuda_bf16.h>
 
-#include "async_copy.cuh"
+#include "gauss_warp.cuh"
 #include "internal.h"
 
 namespace exfem {
@@ -40,12 +40,10 @@ template <int ET, bool J2, int MODE, class OutT>
 struct StiffSmem {
   using Tr = ElemTraits<ET>;
   static constexpr int NN = Tr::nnode, NG = Tr::ngp, ND = 3 * NN, EPW = 32 / NG;
-  static constexpr int XS = 3 * NN + 1;  // odd stride: the elements' broadcasts fall into different banks
   union {                  // node values (first part), then the matrix being put together
     alignas(16) OutT stage[MODE == 0 ? ND * ND : 8];
     struct {
-      double x[EPW * XS];
-      double u[J2 ? EPW * XS : 1];
+      NodeSmem<ET, J2> nd;
       double st[J2 ? 32 * 19 : 1];  // Gauss-point states: the lanes' odd stride of 19 meets no bank conflict
     };
   };
@@ -77,7 +75,7 @@ stiffness_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __rest
                  const double* __restrict__ lam_e, const double* __restrict__ mu_e, OutT* __restrict__ Ke,
                  double* __restrict__ ediag, const int32_t* __restrict__ tpos, int tile, int bulk) {
   using S = StiffSmem<ET, J2, MODE, OutT>;
-  constexpr int NN = S::NN, NG = S::NG, ND = S::ND, EPW = S::EPW, XS = S::XS;
+  constexpr int NN = S::NN, NG = S::NG, ND = S::ND, EPW = S::EPW, XS = DnTable<ET>::XS;
   constexpr int NT = NN > 8 ? 2 : 1, KS = NG / 4;  // node tiles per side, matrix steps over the Gauss points
   constexpr bool BBAR = ET == EXFEM_C3D8;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -85,10 +83,7 @@ stiffness_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __rest
   constexpr int TAB = (NG * XS + 15) / 16 * 16;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   S& sm = reinterpret_cast<S*>(tab + TAB)[warp];
-  for (int k = threadIdx.x; k < NG * 3 * NN; k += 32 * NW) {
-    const int g = k / (3 * NN), r = k % (3 * NN);
-    tab[g * XS + r] = elem_dN(ET, g, r / 3, r % 3);
-  }
+  for (int k = threadIdx.x; k < NG * XS; k += 32 * NW) tab[k] = dn_table<ET>()[k];
   __syncthreads();
   const int row = lane >> 2, q = lane & 3;  // this lane's row and Gauss point (matrix A), or column pair (C)
   double dNl[KS][NT][3];
@@ -109,54 +104,21 @@ stiffness_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __rest
   if (J2 && !tan_in && st_old) {
     for (int k = lane; k < cnt * NG * 19; k += 32) cp_async<8>(sm.st + k, st_old + e0 * (NG * 19) + k, 8);
   }
-  for (int k = lane; k < cnt * NN; k += 32) {
-    const int64_t n3 = 3 * (int64_t)conn[e0 * NN + k];
-    const int o = (k / NN) * XS + 3 * (k % NN);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      sm.x[o + c] = X[n3 + c];
-      if constexpr (J2) sm.u[o + c] = u ? u[n3 + c] : 0.0;
-    }
-  }
+  const int le = lane / NG, g = lane % NG;
+  gather_nodes<ET, J2>(sm.nd, X, conn, u, e0 + (le < cnt ? le : 0), cnt, [&](int el) { return e0 + el; });
   if constexpr (J2) cp_async_wait_all();
   __syncwarp();
 
   // ---- one lane per Gauss point: geometry and material
-  const int le = lane / NG, g = lane % NG;
   bool plastic = false;
   if (le < cnt) {
     const int64_t e = e0 + le;
     const bool own = lam_e != nullptr;  // per-element Lame parameters override the material's
     const double lam_k = own ? lam_e[e] : mat.lam, mu_k = own ? mu_e[e] : mat.mu;
-    double J[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    const double* dn = tab + g * XS;
-    const double *xe = sm.x + le * XS, *ue = sm.u + le * XS;
-#pragma unroll
-    for (int b = 0; b < NN; ++b)
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          J[3 * c + i] += xe[3 * b + c] * dn[3 * b + i];
-          if constexpr (J2) G[3 * c + i] += ue[3 * b + c] * dn[3 * b + i];
-        }
-    double iJ[9], iJ0[9], G0[9];
+    double J[9], G[9], J0[9], G0[9], iJ[9], iJ0[9];
+    gauss_gradients<ET, J2>(sm.nd, tab, le, g, J, G, J0, G0);
     const double detJ = inv3(J, iJ);
     if constexpr (BBAR) {
-      double J0[9];
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          double sx = 0.0, su = 0.0;
-#pragma unroll
-          for (int b = 0; b < 8; ++b) {
-            sx += hex_sign(b, i) > 0 ? xe[3 * b + c] : -xe[3 * b + c];
-            if constexpr (J2) su += hex_sign(b, i) > 0 ? ue[3 * b + c] : -ue[3 * b + c];
-          }
-          J0[3 * c + i] = 0.125 * sx;
-          G0[3 * c + i] = 0.125 * su;
-        }
       inv3(J0, iJ0);
       if (g == 0)
 #pragma unroll
@@ -172,9 +134,12 @@ stiffness_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __rest
         double H[9], sig[6], st[19];
         matmul3(G, iJ, H);
         if constexpr (BBAR) {
-          double H0[9];
-          matmul3(G0, iJ0, H0);
-          const double bb = ((H0[0] + H0[4] + H0[8]) - (H[0] + H[4] + H[8])) * (1.0 / 3.0);
+          double tr0 = 0.0;
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) tr0 += G0[3 * c + i] * iJ0[3 * i + c];
+          const double bb = (tr0 - (H[0] + H[4] + H[8])) * (1.0 / 3.0);
           H[0] += bb;
           H[4] += bb;
           H[8] += bb;
@@ -367,7 +332,7 @@ int stiffness_go(exfem_block_s* b, const double* u, const double* st_old, const 
                  double* ediag, cudaStream_t s) {
   using S = StiffSmem<ET, J2, MODE, OutT>;
   constexpr int NW = 4;
-  constexpr size_t smem = (size_t)((S::NG * S::XS + 15) / 16 * 16) * sizeof(double) + NW * sizeof(S);
+  constexpr size_t smem = (size_t)((S::NG * DnTable<ET>::XS + 15) / 16 * 16) * sizeof(double) + NW * sizeof(S);
   auto kern = stiffness_kernel<ET, J2, MODE, OutT, NW>;
   if constexpr (smem > 48 * 1024)
     EX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
