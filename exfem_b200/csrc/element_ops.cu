@@ -10,37 +10,45 @@ namespace exfem {
 
 // ---------------------------------------------------------------- assembly
 // f[3n+c] = sum over the gather plan of node n (reference order); optional opA
-// finalisation y = fixed ? v : sum.
-__global__ void gather_assemble_kernel(int64_t nn, int vmax, const int32_t* __restrict__ plan,
-                                       int64_t sentinel, const double* __restrict__ ys,
-                                       double* __restrict__ f, const uint8_t* __restrict__ fixed,
-                                       const double* __restrict__ v, const int* __restrict__ skip) {
+// finalisation y = fixed ? v : sum.  One thread per degree of freedom: the three of a
+// node read neighbouring entries, and eight plan slots and their entries are requested
+// before any is added (in the plan's order), because the kernel is bound by the latency
+// of the plan -> entry chain: one thread per node with one slot in flight took 10 us
+// for 44,541 nodes of C3D8 and 27 us for 176,715 of C3D10.
+__global__ void __launch_bounds__(256)
+gather_assemble_kernel(int64_t ndof, int vmax, const int32_t* __restrict__ plan, int32_t sentinel,
+                       const double* __restrict__ ys, double* __restrict__ f, const uint8_t* __restrict__ fixed,
+                       const double* __restrict__ v, const int* __restrict__ skip) {
+  constexpr int K = 8;
   if (skip && *skip) return;
-  const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (n >= nn) return;
-  double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+  const int64_t d = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (d >= ndof) return;
+  const int64_t n = d / 3;
+  const int c = (int)(d - 3 * n);
   const int32_t* row = plan + n * vmax;
-  for (int k = 0; k < vmax; ++k) {
-    const int64_t slot = row[k];
-    if (slot == sentinel) break;
-    s0 += ys[3 * slot];
-    s1 += ys[3 * slot + 1];
-    s2 += ys[3 * slot + 2];
-  }
-  const double s[3] = {s0, s1, s2};
+  const bool pass = v && fixed && fixed[d];
+  double s = 0.0;
+  for (int k0 = 0; k0 < vmax; k0 += K) {
+    int32_t slot[K];
+    double w[K];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const int64_t d = 3 * n + c;
-    f[d] = (v && fixed && fixed[d]) ? v[d] : s[c];
+    for (int k = 0; k < K; ++k) slot[k] = k0 + k < vmax ? row[k0 + k] : sentinel;
+#pragma unroll
+    for (int k = 0; k < K; ++k) w[k] = slot[k] != sentinel ? ys[3 * (int64_t)slot[k] + c] : 0.0;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (slot[k] != sentinel) s += w[k];
+    if (slot[K - 1] == sentinel) break;  // slots are listed without gaps
   }
+  f[d] = pass ? v[d] : s;
 }
 
 int launch_gather_assemble(exfem_block_s* b, const double* ys, double* f, const double* v_opa,
                            const int* skip, cudaStream_t s) {
   if (b->nn == 0) return EXFEM_OK;
   const int threads = 256;
-  gather_assemble_kernel<<<(unsigned)((b->nn + threads - 1) / threads), threads, 0, s>>>(
-      b->nn, b->vmax, b->plan.p, b->ne * b->nnode, ys, f, v_opa ? b->fixed.p : nullptr, v_opa, skip);
+  gather_assemble_kernel<<<(unsigned)((b->ndof() + threads - 1) / threads), threads, 0, s>>>(
+      b->ndof(), b->vmax, b->plan.p, (int32_t)(b->ne * b->nnode), ys, f, v_opa ? b->fixed.p : nullptr, v_opa, skip);
   EX_LAUNCH_CHECK();
   return EXFEM_OK;
 }
