@@ -228,37 +228,80 @@ int launch_geo_stiffness(exfem_block_s* b, const double* S, double* Kg, cudaStre
 }
 
 // ---------------------------------------------------------------- stored-Ke products
-// ys[e, r] = sum_j Ke[e, r, j] * (free*v)[dofs[e, j]]   (one thread per element row)
-__global__ void ebe_rows_kernel(int64_t ne, int nnode, const int32_t* __restrict__ conn,
-                                const double* __restrict__ Ke, const double* __restrict__ v,
-                                const uint8_t* __restrict__ fixed, double* __restrict__ ys,
-                                const int* __restrict__ skip) {
+// ys[e, r] = sum_j Ke[e, r, j] * (free*v)[dofs[e, j]]
+//
+// Bound by streaming Ke.  One warp per element: four lanes share a row and read it in
+// 16-byte pieces 64 contiguous bytes at a time (8 rows of an element per load
+// instruction, every sector whole), all pieces of an element requested before the
+// first is used; the lanes' v come from one gather of the element's DOFs by shuffles,
+// and a row is summed over its four lanes.  40,641 C3D8 (187 MB of Ke) on B200: 30 us
+// against 77 us for one thread per row, whose loads were a row apart.
+template <int ET, bool VEC>
+__global__ void __launch_bounds__(256)
+ebe_rows_kernel(int64_t ne, const int32_t* __restrict__ conn, const double* __restrict__ Ke,
+                const double* __restrict__ v, const uint8_t* __restrict__ fixed, double* __restrict__ ys,
+                const int* __restrict__ skip) {
+  constexpr int NN = ElemTraits<ET>::nnode, ND = 3 * NN, NP = ND / 2;  // pieces of 16 bytes per row
+  constexpr int RP = (ND + 7) / 8, PL = (NP + 3) / 4;                  // passes over the rows, pieces per lane
   if (skip && *skip) return;
-  const int nd = 3 * nnode;
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= ne * nd) return;
-  const int64_t e = t / nd;
-  const int r = (int)(t - e * nd);
-  const double* K = Ke + e * nd * nd + (int64_t)r * nd;
-  double s = 0.0;
-  for (int a = 0; a < nnode; ++a) {
-    const int64_t n3 = 3 * (int64_t)conn[e * nnode + a];
-    for (int c = 0; c < 3; ++c) {
-      const double vv = (fixed && fixed[n3 + c]) ? 0.0 : v[n3 + c];
-      s += K[3 * a + c] * vv;
+  const int lane = threadIdx.x & 31, row = lane >> 2, q = lane & 3;
+  const int64_t e = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  if (e >= ne) return;
+  const double* K = Ke + e * (ND * ND);
+  double2 k[RP][PL];
+#pragma unroll
+  for (int r = 0; r < RP; ++r)
+#pragma unroll
+    for (int p = 0; p < PL; ++p) {
+      const int i = 8 * r + row, j = q + 4 * p;
+      k[r][p] = make_double2(0.0, 0.0);
+      if (i < ND && j < NP) {
+        const double* src = K + i * ND + 2 * j;
+        if constexpr (VEC) k[r][p] = __ldcs(reinterpret_cast<const double2*>(src));
+        else k[r][p] = make_double2(src[0], src[1]);
+      }
     }
+  double vl = 0.0;
+  if (lane < ND) {
+    const int64_t d = 3 * (int64_t)conn[e * NN + lane / 3] + lane % 3;
+    vl = (fixed && fixed[d]) ? 0.0 : v[d];
   }
-  ys[t] = s;
+  double s[RP];
+#pragma unroll
+  for (int r = 0; r < RP; ++r) s[r] = 0.0;
+#pragma unroll
+  for (int p = 0; p < PL; ++p) {
+    const double va = __shfl_sync(0xffffffffu, vl, 2 * (q + 4 * p)), vb = __shfl_sync(0xffffffffu, vl, 2 * (q + 4 * p) + 1);
+    const bool in = q + 4 * p < NP;
+#pragma unroll
+    for (int r = 0; r < RP; ++r)
+      if (in) s[r] = fma(k[r][p].y, vb, fma(k[r][p].x, va, s[r]));
+  }
+#pragma unroll
+  for (int r = 0; r < RP; ++r) {
+    s[r] += __shfl_xor_sync(0xffffffffu, s[r], 1);
+    s[r] += __shfl_xor_sync(0xffffffffu, s[r], 2);
+    if (q == 0 && 8 * r + row < ND) ys[e * ND + 8 * r + row] = s[r];
+  }
 }
 
 int launch_ebe_matvec(exfem_block_s* b, const double* Ke, const double* v, double* y,
                       const int* skip, cudaStream_t s, bool bc) {
   int st;
   if (b->ys.n < (size_t)(b->ne * b->nnode * 3) && (st = b->ys.alloc(b->ne * b->nnode * 3))) return st;
-  const int64_t rows = b->ne * b->nnode * 3;
-  if (rows) {
-    ebe_rows_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, s>>>(b->ne, b->nnode, b->conn.p, Ke, v,
-                                                                   bc ? b->fixed.p : nullptr, b->ys.p, skip);
+  if (b->ne) {
+    const unsigned grid = (unsigned)((b->ne + 7) / 8);
+    const uint8_t* fx = bc ? b->fixed.p : nullptr;
+    const bool vec = (uintptr_t)Ke % 16 == 0;  // element matrices are multiples of 16 bytes
+#define EXF_ROWS(ET, VEC) ebe_rows_kernel<ET, VEC><<<grid, 256, 0, s>>>(b->ne, b->conn.p, Ke, v, fx, b->ys.p, skip)
+    if (b->etype == EXFEM_C3D8) {
+      if (vec) EXF_ROWS(EXFEM_C3D8, true);
+      else EXF_ROWS(EXFEM_C3D8, false);
+    } else {
+      if (vec) EXF_ROWS(EXFEM_C3D10, true);
+      else EXF_ROWS(EXFEM_C3D10, false);
+    }
+#undef EXF_ROWS
     EX_LAUNCH_CHECK();
   }
   return launch_gather_assemble(b, b->ys.p, y, bc ? v : nullptr, skip, s);
