@@ -556,19 +556,13 @@ int exfem_tangent_diagonal(exfem_block b, double* diag, void* stream) {
 int exfem_ebe_matvec_bf16_multi(exfem_block b, const void* Ke_bf16, int nrhs, const float* V, float* Y,
                                 int apply_bc, void* stream) {
   EX_ARG(b && (b->ne == 0 || Ke_bf16) && V && Y, "NULL argument");
-  StreamGuard g;
-  int s;
-  if ((s = g.init(stream))) return s;
-  return launch_ebe_matvec_tc(b, (const __nv_bfloat16*)Ke_bf16, nrhs, V, Y, g.work, apply_bc != 0);
+  return launch_ebe_matvec_tc(b, (const __nv_bfloat16*)Ke_bf16, nrhs, V, Y, as_stream(stream), apply_bc != 0);
 }
 
 int exfem_ebe_matvec_multi(exfem_block b, const void* Ke, int ke_dtype, int nrhs, const void* V, void* Y,
                            int apply_bc, void* stream) {
   EX_ARG(b && (b->ne == 0 || Ke) && V && Y, "NULL argument");
-  StreamGuard g;
-  int s;
-  if ((s = g.init(stream))) return s;
-  return launch_ebe_matvec_multi(b, Ke, ke_dtype, nrhs, V, Y, apply_bc != 0, g.work);
+  return launch_ebe_matvec_multi(b, Ke, ke_dtype, nrhs, V, Y, apply_bc != 0, as_stream(stream));
 }
 
 int exfem_multi_pcg(exfem_block b, const double* Ke, int nrhs, const double* B, double* X, double tol, int maxiter,
@@ -593,10 +587,7 @@ int exfem_ebe_diagonal(exfem_block b, const double* Ke, double* diag, void* stre
 
 int exfem_geometric_stiffness(exfem_block b, const double* S, double* Kg, void* stream) {
   EX_ARG(b && (S || b->ne == 0) && (Kg || b->ne == 0), "NULL argument");
-  StreamGuard g;
-  int st;
-  if ((st = g.init(stream))) return st;
-  return launch_geo_stiffness(b, S, Kg, g.work);
+  return launch_geo_stiffness(b, S, Kg, as_stream(stream));
 }
 
 int exfem_stresses(exfem_block b, const double* u, const double* state, double* S, double* mises, double* peeq,
