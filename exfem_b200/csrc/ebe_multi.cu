@@ -12,18 +12,16 @@
 // Per element the work is Ke (nd x nd) times U_e (nd x nrhs): 2 FMA per byte of
 // BF16 Ke at four right-hand sides, far below what the tensor cores need to be the
 // bound, so the contraction runs on the CUDA cores and the kernel is bound by
-// streaming Ke.  Each warp takes elements in turn (grid-stride, two per pass for BF16
-// and FP32 Ke): it gathers their nodal values (prescribed DOFs zeroed) into its
-// shared-memory slice, lane i < nd multiplies row i of Ke — read with the widest
-// aligned loads — by them (broadcast reads) and stores the nrhs results of its row;
-// the element rows are then summed per node through the gather plan in the
-// reference's order (gfem/model.py:241-267) and opA's prescribed rows applied
+// streaming Ke.  The element rows are then summed per node through the gather plan in
+// the reference's order (gfem/model.py:241-267) and opA's prescribed rows applied
 // (gather_multi_kernel).
 #include <cuda_bf16.h>
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
+#include "async_copy.cuh"
 #include "internal.h"
 #include "solver.h"
 
@@ -37,256 +35,249 @@ template <>
 __device__ __forceinline__ float to_acc<__nv_bfloat16>(__nv_bfloat16 v, float) { return __bfloat162float(v); }
 __device__ __forceinline__ double to_acc(double v, double) { return v; }
 
-// N values of T at p into registers with the widest loads the alignment A allows
-template <class T, int N, int A>
-__device__ __forceinline__ void ld_row(const T* __restrict__ p, T (&o)[N]) {
-  constexpr int BYTES = N * (int)sizeof(T);
-  if constexpr (A % 16 == 0 && BYTES % 16 == 0) {
-#pragma unroll
-    for (int i = 0; i < BYTES / 16; ++i) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(p) + i);
-      memcpy(reinterpret_cast<char*>(o) + 16 * i, &v, 16);
-    }
-  } else if constexpr (A % 8 == 0 && BYTES % 8 == 0) {
-#pragma unroll
-    for (int i = 0; i < BYTES / 8; ++i) {
-      const uint2 v = __ldg(reinterpret_cast<const uint2*>(p) + i);
-      memcpy(reinterpret_cast<char*>(o) + 8 * i, &v, 8);
-    }
-  } else if constexpr (A % 4 == 0 && BYTES % 4 == 0) {
-#pragma unroll
-    for (int i = 0; i < BYTES / 4; ++i) {
-      const unsigned v = __ldg(reinterpret_cast<const unsigned*>(p) + i);
-      memcpy(reinterpret_cast<char*>(o) + 4 * i, &v, 4);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < N; ++i) o[i] = p[i];
-  }
-}
-
-// byte alignment of row i of a 256-byte aligned array of rows of N values of T
-template <class T, int N>
-constexpr int row_align() {
-  return (N * (int)sizeof(T)) % 16 == 0 ? 16
-         : (N * (int)sizeof(T)) % 8 == 0 ? 8
-         : (N * (int)sizeof(T)) % 4 == 0 ? 4
-                                         : 2;
-}
-
-constexpr int MW = 8;  // warps per CTA
-
 }  // namespace
 
 // ys[(e*nd + i)*NR + r] = sum_j Ke[e, i, j] * (free * V)[dof(e, j), r]
 //
-// Each warp takes EP elements per pass (EP = 2 for BF16 / FP32 Ke, 1 for FP64): the
-// Ke rows of all of them are requested first, then their nodal values are gathered
-// together (16-byte vectors of right-hand sides where nrhs allows), so that every
-// lane has EP rows and EP gathers in flight at once.  FP32 products of an even
-// number of right-hand sides issue packed FFMA2 (two right-hand sides per
-// instruction, each rounded as its own FMA).
+// One warp takes 4 C3D8 or 3 C3D10, one lane per element node: the lane forms the
+// node's three rows, so that a value of U read from shared memory serves three rows of
+// up to four elements at once (their lanes read different elements' values together).
+// Ke comes into shared memory by bulk copies, in the same order as it is stored where
+// the lanes' rows then lie in different banks (3 rows = an odd number of access
+// widths), else with a padded copy per lane; the element values of V are gathered in
+// 16-byte vectors meanwhile.  The rows leave through shared memory as one bulk store.
+// B200, 131,072 C3D8 in BF16, four right-hand sides: 46 us; one lane per row with
+// every value of U broadcast to one element's lanes took 55 us (the L1 pipe 79% busy:
+// 87 wavefronts an element against 27 here).
 template <int ET, int NR, class KT, class VT>
-__global__ void __launch_bounds__(32 * MW)
-ebe_multi_kernel(int64_t ne, const int32_t* __restrict__ conn, const KT* __restrict__ Ke,
-                 const VT* __restrict__ V, const uint8_t* __restrict__ fixed, VT* __restrict__ ys, int vecv) {
-  constexpr int NN = ElemTraits<ET>::nnode, ND = 3 * NN;
-  constexpr int EP = sizeof(KT) <= 4 ? 2 : 1;
-  constexpr int W = (NR * sizeof(VT)) % 16 == 0 ? 16 / (int)sizeof(VT) : 1;  // values per gathered vector
-  constexpr int NV = ND * NR / W;
-  constexpr bool PAIRED = sizeof(VT) == 4 && NR % 2 == 0;
-  __shared__ __align__(16) VT us[MW][EP][ND * NR];
+struct MultiSmem {
+  using Ke = KT;
+  static constexpr int NN = ElemTraits<ET>::nnode, ND = 3 * NN, EPW = 32 / NN;
+  static constexpr int CHUNK = 3 * ND * (int)sizeof(KT);  // a lane's rows
+  static constexpr int AW = CHUNK % 16 == 0 ? 16 : (CHUNK % 8 == 0 ? 8 : 4);
+  static constexpr bool PAD = (CHUNK / AW) % 2 == 0;      // rows would share banks: padded copies
+  static constexpr int KP = PAD ? CHUNK + 16 : CHUNK;
+  static constexpr int W = 16 / (int)sizeof(VT), NRP = (NR + W - 1) / W * W;
+  static constexpr int US = ND * NRP + W;                 // element stride of U: different banks
+  static constexpr int KB = (EPW * NN * KP + 15) / 16 * 16;
+  alignas(16) unsigned char k[KB];
+  alignas(16) VT u[EPW * US];                             // U, then the rows
+  uint64_t bar;
+};
+
+// right-hand sides R0 .. R0 + RG - 1 of a node's three rows; kr: the rows of Ke, ue: the
+// element's values
+template <int R0, int RG, class S, class VT>
+__device__ __forceinline__ void node_rows(const unsigned char* kr, const VT* ue, VT (&y)[3][S::NRP]) {
+  using KT = typename S::Ke;
+  constexpr int ND = S::ND, W = S::W, NRP = S::NRP, AW = S::AW, CW = AW / (int)sizeof(KT);  // columns per read of Ke
+  static_assert(RG % W == 0 && R0 + RG <= NRP, "whole vectors of right-hand sides");
+  VT acc[3][RG];
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int j = 0; j < RG; ++j) acc[r][j] = VT(0);
+#pragma unroll
+  for (int c0 = 0; c0 < ND; c0 += CW) {
+    KT k[3][CW];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      using L = std::conditional_t<AW == 16, uint4, std::conditional_t<AW == 8, uint2, unsigned>>;
+      const L t = *reinterpret_cast<const L*>(kr + (r * ND + c0) * sizeof(KT));
+      memcpy(k[r], &t, AW);
+    }
+#pragma unroll
+    for (int c = 0; c < CW; ++c) {
+      VT u[RG];
+#pragma unroll
+      for (int h = 0; h < RG / W; ++h) {
+        const uint4 t = *reinterpret_cast<const uint4*>(ue + (c0 + c) * NRP + R0 + h * W);
+        memcpy(u + h * W, &t, 16);
+      }
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const VT kc = to_acc(k[r][c], VT(0));
+        if constexpr (sizeof(VT) == 4) {
+#pragma unroll
+          for (int j = 0; j < RG; j += 2) {
+            const float2 t =
+                __ffma2_rn(make_float2(kc, kc), make_float2(u[j], u[j + 1]), make_float2(acc[r][j], acc[r][j + 1]));
+            acc[r][j] = t.x;
+            acc[r][j + 1] = t.y;
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < RG; ++j) acc[r][j] += kc * u[j];
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int j = 0; j < RG; ++j) y[r][R0 + j] = acc[r][j];
+}
+
+template <int ET, int NR, class KT, class VT, int NW>
+__global__ void __launch_bounds__(32 * NW)
+ebe_multi_kernel(int64_t ne, const int32_t* __restrict__ conn, const KT* __restrict__ Ke, const VT* __restrict__ V,
+                 const uint8_t* __restrict__ fixed, VT* __restrict__ ys, int vecv, int aligned, int* __restrict__ err) {
+  using S = MultiSmem<ET, NR, KT, VT>;
+  constexpr int NN = S::NN, ND = S::ND, EPW = S::EPW, W = S::W, NRP = S::NRP;
+  constexpr int EB = ND * ND * (int)sizeof(KT);  // bytes of an element's matrix
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t stride = (int64_t)gridDim.x * MW;
-  for (int64_t e0 = (int64_t)blockIdx.x * MW + warp; e0 < ne; e0 += EP * stride) {
-    KT row[EP][ND];
-#pragma unroll
-    for (int p = 0; p < EP; ++p) {
-      const int64_t e = e0 + p * stride;
-      if (e < ne && lane < ND) ld_row<KT, ND, row_align<KT, ND>()>(Ke + (e * ND + lane) * ND, row[p]);
-    }
-#pragma unroll
-    for (int p = 0; p < EP; ++p) {
-      const int64_t e = e0 + p * stride;
-      if (e < ne) {
-        for (int q = lane; q < NV; q += 32) {
-          const int i = (q * W) / NR, r = (q * W) % NR;
-          const int64_t d = 3 * (int64_t)__ldg(conn + e * NN + i / 3) + i % 3;
-          const bool off = fixed && __ldg(fixed + d);
-          if constexpr (W > 1) {
-            uint4 v;
-            if (vecv) {  // V 16-byte aligned (checked on the host)
-              v = __ldg(reinterpret_cast<const uint4*>(V + d * NR + r));
-            } else {
-              VT t[W];
-#pragma unroll
-              for (int k = 0; k < W; ++k) t[k] = __ldg(V + d * NR + r + k);
-              memcpy(&v, t, 16);
-            }
-            if (off) v = make_uint4(0, 0, 0, 0);
-            *reinterpret_cast<uint4*>(&us[warp][p][q * W]) = v;
-          } else {
-            const VT v = __ldg(V + d * NR + r);
-            us[warp][p][q] = off ? VT(0) : v;
-          }
-        }
-      }
+  S& sm = reinterpret_cast<S*>(smem_raw)[warp];
+  const int64_t e0 = ((int64_t)blockIdx.x * NW + warp) * EPW;
+  if (e0 >= ne) return;
+  const int cnt = ne - e0 < EPW ? (int)(ne - e0) : EPW;
+  const int el = lane / NN, node = lane - el * NN;
+  const bool on = el < cnt;  // C3D10: el = 3 for the two spare lanes
+  // ---- Ke: bulk copies need 16-byte boundaries and sizes
+  const unsigned char* src = reinterpret_cast<const unsigned char*>(Ke) + e0 * EB;
+  const bool bulk = aligned && (e0 * EB) % 16 == 0 && (cnt * EB) % 16 == 0;
+  if (bulk) {
+    if (lane == 0) {
+      mbar_init(&sm.bar, 1);
+      fence_mbar_init();
+      mbar_expect_tx(&sm.bar, cnt * EB);
     }
     __syncwarp();
+    if constexpr (S::PAD) {
+      if (on) bulk_g2s(sm.k + lane * S::KP, src + lane * S::CHUNK, S::CHUNK, &sm.bar);
+    } else {
+      if (lane == 0) bulk_g2s(sm.k, src, cnt * EB, &sm.bar);
+    }
+  } else {
+    for (int i = lane; i < cnt * EB / 4; i += 32)
+      cp_async<4>(sm.k + (S::PAD ? i * 4 / S::CHUNK * (S::KP - S::CHUNK) : 0) + i * 4, src + i * 4, 4);
+  }
+  // ---- element values of V, prescribed DOFs zeroed
 #pragma unroll
-    for (int p = 0; p < EP; ++p) {
-      const int64_t e = e0 + p * stride;
-      if (e < ne && lane < ND) {
-        const VT* u = us[warp][p];
-        VT y[NR];
-        if constexpr (PAIRED) {
-          float2 y2[NR / 2];
+  for (int i0 = 0; i0 < EPW * ND; i0 += 32) {
+    const int i = i0 + lane;
+    if (i < cnt * ND) {
+      const int64_t d = 3 * (int64_t)__ldg(conn + e0 * NN + i / 3) + i % 3;
+      const bool off = fixed && __ldg(fixed + d);
+      const VT* v = V + d * NR;
+      VT* dst = sm.u + (i / ND) * S::US + (i % ND) * NRP;
+      if (NR % W == 0 && vecv) {  // V 16-byte aligned (checked on the host)
 #pragma unroll
-          for (int j = 0; j < NR / 2; ++j) y2[j] = make_float2(0.f, 0.f);
-#pragma unroll
-          for (int c = 0; c < ND; ++c) {
-            const float k = to_acc(row[p][c], 0.f);
-            const float2 k2 = make_float2(k, k);
-            const float2* u2 = reinterpret_cast<const float2*>(u + c * NR);
-#pragma unroll
-            for (int j = 0; j < NR / 2; ++j) y2[j] = __ffma2_rn(k2, u2[j], y2[j]);
-          }
-#pragma unroll
-          for (int j = 0; j < NR / 2; ++j) {
-            y[2 * j] = y2[j].x;
-            y[2 * j + 1] = y2[j].y;
-          }
-        } else {
-#pragma unroll
-          for (int r = 0; r < NR; ++r) y[r] = VT(0);
-#pragma unroll
-          for (int c = 0; c < ND; ++c) {
-            const VT k = to_acc(row[p][c], VT(0));
-#pragma unroll
-            for (int r = 0; r < NR; ++r) y[r] += k * u[c * NR + r];
-          }
+        for (int h = 0; h < NRP / W; ++h) {
+          uint4 t = __ldg(reinterpret_cast<const uint4*>(v) + h);
+          if (off) t = make_uint4(0, 0, 0, 0);
+          reinterpret_cast<uint4*>(dst)[h] = t;
         }
-        VT* out = ys + (e * ND + lane) * NR;
-        if constexpr ((NR * sizeof(VT)) % 16 == 0) {
+      } else {
 #pragma unroll
-          for (int r = 0; r < NR; r += 16 / (int)sizeof(VT)) {
-            uint4 w;
-            memcpy(&w, y + r, 16);
-            *reinterpret_cast<uint4*>(out + r) = w;
-          }
-        } else {
-#pragma unroll
-          for (int r = 0; r < NR; ++r) out[r] = y[r];
-        }
+        for (int j = 0; j < NRP; ++j) dst[j] = j < NR && !off ? __ldg(v + j) : VT(0);
       }
     }
+  }
+  if (bulk) {
+    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&sm.bar, 0, err))) return;
+  } else {
+    cp_async_wait_all();
+  }
+  __syncwarp();
+  // ---- the node's three rows, at most eight FP64 right-hand sides at a time (registers)
+  const unsigned char* kr = sm.k + (on ? lane : 0) * S::KP;
+  const VT* ue = sm.u + (on ? el : 0) * S::US;
+  constexpr int R1 = sizeof(VT) == 8 && NRP > 8 ? 8 : NRP;
+  VT y[3][NRP];
+  node_rows<0, R1, S>(kr, ue, y);
+  if constexpr (R1 < NRP) node_rows<R1, NRP - R1, S>(kr, ue, y);
+  __syncwarp();  // every lane has read U: its place takes the rows, as they are stored
+  if (on) {
+    VT* o = sm.u + lane * 3 * NR;
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int j = 0; j < NR; j += (NR % W == 0 ? W : 1)) {
+        if constexpr (NR % W == 0) {
+          uint4 t;
+          memcpy(&t, &y[r][j], 16);
+          *reinterpret_cast<uint4*>(o + r * NR + j) = t;
+        } else {
+          o[r * NR + j] = y[r][j];
+        }
+      }
+  }
+  const int bytes = cnt * ND * NR * (int)sizeof(VT);
+  VT* out = ys + e0 * (ND * NR);
+  if (bytes % 16 == 0 && (uintptr_t)out % 16 == 0) {
+    fence_proxy_async();
     __syncwarp();
+    if (lane == 0) {
+      bulk_s2g(out, sm.u, bytes);
+      bulk_commit();
+      bulk_wait_read<0>();
+    }
+  } else {
+    __syncwarp();
+    for (int i = lane; i < cnt * ND * NR; i += 32) out[i] = sm.u[i];
   }
 }
 
 // Y[3n+c, r] = fixed ? V : sum over node n's gather-plan slots of the element rows,
-// the slots in the plan's order; one thread per node and group of four right-hand
-// sides (16-byte loads and stores) for FP32 with nrhs a multiple of 4 and aligned
-// V, Y (vec4), else per node and right-hand side.  The plan entries are read four
-// at a time and the rows of all four slots requested before any is added.
-template <class VT>
-__global__ void __launch_bounds__(256) gather_multi_kernel(int64_t nn, int vmax, int nnode, const int32_t* __restrict__ plan,
-                                    int64_t sentinel, const VT* __restrict__ ys, const uint8_t* __restrict__ fixed,
-                                    const VT* __restrict__ V, int nrhs, VT* __restrict__ Y, int vec4) {
-  constexpr int K = 4;
-  const int nd = 3 * nnode;
+// the slots in the plan's order (slot s holds rows 3s .. 3s+2).  One thread per degree
+// of freedom and group of right-hand sides (four FP32, two FP64: 16 bytes) where their
+// number and the addresses allow it (vec), else one right-hand side; eight plan slots
+// and their rows are requested before any is added.  One thread per node, with three
+// rows of four slots in flight, took 23 us for 140,481 nodes and four FP32 right-hand
+// sides (18 us now).
+template <class VT, int W>
+__global__ void __launch_bounds__(256)
+gather_multi_kernel(int64_t ndof, int vmax, const int32_t* __restrict__ plan, int32_t sentinel,
+                    const VT* __restrict__ ys, const uint8_t* __restrict__ fixed, const VT* __restrict__ V, int nrhs,
+                    VT* __restrict__ Y) {
+  constexpr int K = 8;
+  struct alignas(W * sizeof(VT)) Vec {
+    VT v[W];
+  };
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if constexpr (sizeof(VT) == 4) {
-    if (vec4) {
-      const int nq = nrhs >> 2;
-      if (t >= nn * nq) return;
-      const int64_t n = t / nq;
-      const int r4 = (int)(t - n * nq) * 4;
-      float4 s[3] = {make_float4(0, 0, 0, 0), make_float4(0, 0, 0, 0), make_float4(0, 0, 0, 0)};
-      bool more = true;
-      for (int k0 = 0; k0 < vmax && more; k0 += K) {
-        int64_t sl[K];
+  const int nq = nrhs / W;
+  const int64_t d = nq == 1 ? t : t / nq;
+  if (d >= ndof) return;
+  const int r = (int)(t - d * nq) * W;
+  const int64_t n = d / 3;
+  const int c = (int)(d - 3 * n);
+  const int32_t* row = plan + n * vmax;
+  const bool pass = fixed && fixed[d];
+  Vec s;
 #pragma unroll
-        for (int u = 0; u < K; ++u) sl[u] = k0 + u < vmax ? (int64_t)plan[n * vmax + k0 + u] : sentinel;
-        float4 w[K][3];
+  for (int j = 0; j < W; ++j) s.v[j] = VT(0);
+  for (int k0 = 0; k0 < vmax; k0 += K) {
+    int32_t slot[K];
+    Vec w[K];
 #pragma unroll
-        for (int u = 0; u < K; ++u) {
-          if (sl[u] != sentinel) {
-            const int64_t e = sl[u] / nnode;
-            const int a = (int)(sl[u] - e * nnode);
+    for (int k = 0; k < K; ++k) slot[k] = k0 + k < vmax ? row[k0 + k] : sentinel;
 #pragma unroll
-            for (int c = 0; c < 3; ++c)
-              w[u][c] = *reinterpret_cast<const float4*>(ys + (e * nd + 3 * a + c) * nrhs + r4);
-          }
-        }
+    for (int k = 0; k < K; ++k)
+      if (slot[k] != sentinel) w[k] = *reinterpret_cast<const Vec*>(ys + (3 * (int64_t)slot[k] + c) * nrhs + r);
 #pragma unroll
-        for (int u = 0; u < K; ++u) {
-          if (sl[u] == sentinel) {
-            more = false;
-            break;
-          }
+    for (int k = 0; k < K; ++k)
+      if (slot[k] != sentinel)
 #pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            s[c].x += w[u][c].x;
-            s[c].y += w[u][c].y;
-            s[c].z += w[u][c].z;
-            s[c].w += w[u][c].w;
-          }
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const int64_t d = 3 * n + c;
-        float4* out = reinterpret_cast<float4*>(Y + d * nrhs + r4);
-        *out = (fixed && fixed[d]) ? *reinterpret_cast<const float4*>(V + d * nrhs + r4) : s[c];
-      }
-      return;
-    }
+        for (int j = 0; j < W; ++j) s.v[j] += w[k].v[j];
+    if (slot[K - 1] == sentinel) break;  // slots are listed without gaps
   }
-  if (t >= nn * nrhs) return;
-  const int64_t n = t / nrhs;
-  const int r = (int)(t - n * nrhs);
-  VT s[3] = {VT(0), VT(0), VT(0)};
-  bool more = true;
-  for (int k0 = 0; k0 < vmax && more; k0 += K) {
-    int64_t sl[K];
-#pragma unroll
-    for (int u = 0; u < K; ++u) sl[u] = k0 + u < vmax ? (int64_t)plan[n * vmax + k0 + u] : sentinel;
-    VT w[K][3];
-#pragma unroll
-    for (int u = 0; u < K; ++u) {
-      if (sl[u] != sentinel) {
-        const int64_t e = sl[u] / nnode;
-        const int a = (int)(sl[u] - e * nnode);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) w[u][c] = ys[(e * nd + 3 * a + c) * nrhs + r];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < K; ++u) {
-      if (sl[u] == sentinel) {
-        more = false;
-        break;
-      }
-#pragma unroll
-      for (int c = 0; c < 3; ++c) s[c] += w[u][c];
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const int64_t d = 3 * n + c;
-    Y[d * nrhs + r] = (fixed && fixed[d]) ? V[d * nrhs + r] : s[c];
-  }
+  *reinterpret_cast<Vec*>(Y + d * nrhs + r) = pass ? *reinterpret_cast<const Vec*>(V + d * nrhs + r) : s;
 }
 
 template <class VT>
 int launch_gather_multi(exfem_block_s* b, const VT* ys, const VT* V, VT* Y, int nrhs, bool bc, cudaStream_t s) {
-  // 16-byte accesses need nrhs a multiple of 4 and 16-byte aligned V and Y
-  const int vec4 = sizeof(VT) == 4 && (nrhs & 3) == 0 && ((uintptr_t)V | (uintptr_t)Y) % 16 == 0;
-  const int64_t work = vec4 ? b->nn * (nrhs / 4) : b->nn * nrhs;
-  if (!work) return EXFEM_OK;
-  gather_multi_kernel<VT><<<(unsigned)((work + 255) / 256), 256, 0, s>>>(
-      b->nn, b->vmax, b->nnode, b->plan.p, b->ne * b->nnode, ys, bc ? b->fixed.p : nullptr, V, nrhs, Y, vec4);
+  constexpr int W = 16 / (int)sizeof(VT);
+  if (!b->nn) return EXFEM_OK;
+  const uint8_t* fx = bc ? b->fixed.p : nullptr;
+  const int32_t sentinel = (int32_t)(b->ne * b->nnode);
+  const bool vec = nrhs % W == 0 && ((uintptr_t)V | (uintptr_t)Y | (uintptr_t)ys) % 16 == 0;
+  const int64_t work = b->ndof() * (vec ? nrhs / W : nrhs);
+  const unsigned grid = (unsigned)((work + 255) / 256);
+  if (vec)
+    gather_multi_kernel<VT, W><<<grid, 256, 0, s>>>(b->ndof(), b->vmax, b->plan.p, sentinel, ys, fx, V, nrhs, Y);
+  else
+    gather_multi_kernel<VT, 1><<<grid, 256, 0, s>>>(b->ndof(), b->vmax, b->plan.p, sentinel, ys, fx, V, nrhs, Y);
   EX_LAUNCH_CHECK();
   return EXFEM_OK;
 }
@@ -297,17 +288,28 @@ template int launch_gather_multi<double>(exfem_block_s*, const double*, const do
 
 namespace {
 
+template <int ET, int NR, class KT, class VT>
+int multi_go(exfem_block_s* b, const KT* Ke, const VT* V, VT* ys, const uint8_t* fx, cudaStream_t s) {
+  using S = MultiSmem<ET, NR, KT, VT>;
+  constexpr int NW = sizeof(S) > 16 * 1024 ? 2 : 4;  // small blocks where a warp's share is large
+  constexpr size_t smem = NW * sizeof(S);
+  constexpr int64_t per = NW * S::EPW;
+  auto kern = ebe_multi_kernel<ET, NR, KT, VT, NW>;
+  if constexpr (smem > 48 * 1024)
+    EX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  EX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  kern<<<(unsigned)((b->ne + per - 1) / per), 32 * NW, smem, s>>>(b->ne, b->conn.p, Ke, V, fx, ys,
+                                                                   (uintptr_t)V % 16 == 0, (uintptr_t)Ke % 16 == 0,
+                                                                   b->dev_err.p);
+  EX_LAUNCH_CHECK();
+  return EXFEM_OK;
+}
+
 template <int ET, class KT, class VT>
 int multi_launch(exfem_block_s* b, const KT* Ke, int nrhs, const VT* V, VT* ys, const uint8_t* fx, cudaStream_t s) {
-  int dev, nsm;
-  EX_CUDA(cudaGetDevice(&dev));
-  EX_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((b->ne + MW - 1) / MW, (int64_t)nsm * 8));
-  const int vecv = (uintptr_t)V % 16 == 0;  // 16-byte gathers of V need it aligned
-#define EXF_MULTI(NR)                                                                                   \
-  case NR:                                                                                              \
-    ebe_multi_kernel<ET, NR, KT, VT><<<grid, 32 * MW, 0, s>>>(b->ne, b->conn.p, Ke, V, fx, ys, vecv); \
-    break;
+#define EXF_MULTI(NR) \
+  case NR:            \
+    return multi_go<ET, NR, KT, VT>(b, Ke, V, ys, fx, s);
   switch (nrhs) {
     EXF_MULTI(1) EXF_MULTI(2) EXF_MULTI(3) EXF_MULTI(4) EXF_MULTI(5) EXF_MULTI(6) EXF_MULTI(7) EXF_MULTI(8)
     EXF_MULTI(9) EXF_MULTI(10) EXF_MULTI(11) EXF_MULTI(12) EXF_MULTI(13) EXF_MULTI(14) EXF_MULTI(15)
@@ -317,8 +319,6 @@ int multi_launch(exfem_block_s* b, const KT* Ke, int nrhs, const VT* V, VT* ys, 
       return EXFEM_ERR_ARG;
   }
 #undef EXF_MULTI
-  EX_LAUNCH_CHECK();
-  return EXFEM_OK;
 }
 
 template <class KT, class VT>

@@ -46,3 +46,27 @@ def test_single_product(cuda, kind, ne, offset):
         b.set_fixed(fixed)
         y = b.ebe_matvec(Kd, v.cuda(), apply_bc=bc)
         assert rel_err(y, _reference(b, K, v[:, None], fx)[:, 0]) < 1e-13
+
+
+@pytest.mark.parametrize("kind", ["hex", "tet"])
+@pytest.mark.parametrize("nrhs", [1, 2, 3, 4, 5, 7, 8, 11, 13, 16])
+@pytest.mark.parametrize("ne", [1, 2, 15, 16, 17, 33])
+def test_products_of_several_right_hand_sides(cuda, kind, nrhs, ne):
+    """FP64 bar as above; FP32 accumulation of up to 30 products per row and 24 rows per
+    node: 24 roundings of 6e-8 on sums of unit-variance products, bar 3e-6."""
+    m, b = _block(kind, ne)
+    g = torch.Generator().manual_seed(100 * nrhs + ne)
+    nd = b.etype.nd
+    K = torch.randn(ne, nd, nd, dtype=torch.float64, generator=g)
+    v = torch.randn(m.ndof, nrhs, dtype=torch.float64, generator=g)
+    fixed = np.zeros(m.ndof, bool)
+    fixed[1::5] = True
+    b.set_fixed(fixed)
+    assert rel_err(b.ebe_matvec_multi(K.cuda(), v.cuda()), _reference(b, K, v, fixed)) < 1e-13
+    v32 = v.float()
+    for dt in (torch.float32, torch.bfloat16):
+        Kt = K.to(dt)
+        y = b.ebe_matvec_multi(Kt.cuda(), v32.cuda())
+        assert rel_err(y, _reference(b, Kt.double(), v32.double(), fixed)) < 3e-6
+    none = np.zeros(m.ndof, bool)
+    assert rel_err(b.ebe_matvec_multi(K.cuda(), v.cuda(), apply_bc=False), _reference(b, K, v, none)) < 1e-13
