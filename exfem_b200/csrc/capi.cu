@@ -327,7 +327,9 @@ int exfem_block_create(int etype, const exfem_material* mat, int64_t nn, const d
   if ((s = init_tangent(b.get()))) return s;
   // element-vector scratch (force assembly, stored-Ke products, diagonals); allocated
   // here so that no later call allocates inside a captured CUDA graph
-  if ((s = b->ys.alloc(std::max<int64_t>(ne * b->nnode * 3, 1)))) return s;
+  // (twice where FP64 products need element vectors too: their own, so that a force
+  // evaluation and a solve of one block on two streams share nothing)
+  if ((s = b->ys.alloc(std::max<int64_t>(ne * b->nnode * 3 * (product_by_points(etype, ne) ? 2 : 1), 1)))) return s;
   *out = b.release();
   return EXFEM_OK;
 } catch (...) {

@@ -1,6 +1,6 @@
 // FP64 internal force with the J2 return map and the consistent-tangent data it
-// produces, the tangent data alone, and element-averaged stresses
-// (gfem/model.py:35-81, 129-137, 466-486).
+// produces, the tangent data alone, element-averaged stresses, and the element vectors
+// of the FP64 tangent product (gfem/model.py:35-81, 129-137, 466-490).
 //
 // One warp takes 32 / ngp elements (4 C3D8, 8 C3D10), one lane per Gauss point.  Node
 // values are gathered once per element and Gauss-point states in whole lines into the
@@ -44,19 +44,29 @@ struct ForceSmem {
   uint64_t bar;                  // arrival of the states
 };
 
+// warps an SM holds: the products need few enough registers for 20, except the J2 C3D8's,
+// which would spill (126,000 elements: 80 us at 16, 111 us at 20)
+template <int ET, bool J2, int MODE>
+constexpr int force_warps() {
+  return MODE == FORCE_PRODUCT && !(J2 && ET == EXFEM_C3D8) ? 20 : 16;
+}
+
 template <int ET, bool J2, int MODE, int NW>
-__global__ void __launch_bounds__(32 * NW, 16 / NW)
+__global__ void __launch_bounds__(32 * NW, force_warps<ET, J2, MODE>() / NW)
 force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict__ conn,
              const double* __restrict__ u, const double* __restrict__ scale, const double* st_old, double* st_new,
              double* __restrict__ fe, double* __restrict__ tan64, float* __restrict__ tan32, double* __restrict__ S,
              double* __restrict__ mises, double* __restrict__ peeq, const __grid_constant__ MatDev mat,
              const double* __restrict__ lam_e, const double* __restrict__ mu_e, const int32_t* __restrict__ order,
-             int tile_log2, int bulk, int* __restrict__ err) {
-  using SM = ForceSmem<ET, J2>;
+             int tile_log2, int bulk, int* __restrict__ err, const uint8_t* __restrict__ nf,
+             const int* __restrict__ skip) {
+  using SM = ForceSmem<ET, J2 && MODE != FORCE_PRODUCT>;
   constexpr int NN = SM::NN, NG = SM::NG, ND = SM::ND, EPW = SM::EPW, ST = SM::ST, XS = DnTable<ET>::XS;
   constexpr bool BBAR = SM::BBAR;
   constexpr bool TILED = J2 && MODE != FORCE_STRESS;  // walked in tile order
+  constexpr bool PRODUCT = MODE == FORCE_PRODUCT, OUT = MODE == FORCE_FULL || PRODUCT, STATES = J2 && !PRODUCT;
   constexpr int MT = NN > 8 ? 2 : 1, NTC = (3 * EPW + 7) / 8, KS = NG * 3 / 4 + (BBAR ? 1 : 0);
+  if (PRODUCT && skip && *skip) return;
   __shared__ __align__(16) double tab[NG * XS];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -74,7 +84,7 @@ force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict
   auto elem = [&](int el) { return TILED ? (int64_t)__shfl_sync(0xffffffffu, eid, el * NG) : p0 + el; };
 
   // ---- states (whole elements, one bulk copy each) and node values
-  if (J2 && st_old) {
+  if (STATES && st_old) {
     if (bulk & BULK_OLD) {
       if (lane == 0) {
         mbar_init(&sm.bar, 1);
@@ -92,7 +102,15 @@ force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict
       }
     }
   }
-  gather_nodes<ET, true>(sm.nd, X, conn, u, eid, cnt, elem);
+  gather_nodes<ET, true>(sm.nd, X, conn, u, nf, eid, cnt, elem);
+  // tile_index(pos, 8 g + k, 8 ngp, tile) for a power of two
+  const int64_t tan0 =
+      TILED ? (((pos >> tile_log2) * (NG * 8) + g * 8) << tile_log2) + (pos & ((1 << tile_log2) - 1)) : 0;
+  double tn[8];
+  if constexpr (J2 && PRODUCT) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) tn[k] = tan64[tan0 + (k << tile_log2)];
+  }
   __syncwarp();
 
   // ---- this lane's Gauss point
@@ -113,8 +131,12 @@ force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict
     H[4] += bb;
     H[8] += bb;
   }
-  double sig[6], tn[8], alpha = 0.0;
-  if constexpr (J2) {
+  double sig[6], alpha = 0.0;
+  if constexpr (J2 && PRODUCT) {
+    double e[6];
+    sym_from_grad(H, e);
+    tangent_stress(mat.K, mat.mu, tn, e, sig);
+  } else if constexpr (J2) {
     double* st = sm.st + lane * 19;
     if (!st_old) {
 #pragma unroll
@@ -141,13 +163,11 @@ force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict
   }
   const double vol = (BBAR ? 1.0 : 1.0 / 24.0) * detJ * (MODE != FORCE_STRESS && scale ? scale[eid] : 1.0);
 
-  if constexpr (TILED) {
+  if constexpr (TILED && !PRODUCT) {
     if (valid) {
-      // tile_index(pos, 8 g + k, 8 ngp, tile) for a power of two
-      const int64_t o0 = (((pos >> tile_log2) * (NG * 8) + g * 8) << tile_log2) + (pos & ((1 << tile_log2) - 1));
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const int64_t o = o0 + (k << tile_log2);
+        const int64_t o = tan0 + (k << tile_log2);
         tan64[o] = tn[k];
         tan32[o] = (float)tn[k];
       }
@@ -183,7 +203,7 @@ force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict
     }
   }
 
-  if constexpr (MODE == FORCE_FULL) {
+  if constexpr (OUT) {
     // Q = vol sigma J^-T; under B-bar the deviatoric part, and the mean stress of the
     // element times the gradients at its centre
     double t = 0.0;
@@ -205,7 +225,7 @@ force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict
 #pragma unroll
       for (int i = 0; i < 3; ++i)
         sm.Q[3 * c + i][lane] = r[c][0] * iJ[3 * i] + r[c][1] * iJ[3 * i + 1] + r[c][2] * iJ[3 * i + 2];
-    if (J2 && st_new) {
+    if (STATES && st_new) {
       if (bulk & BULK_NEW) {
         fence_proxy_async();
         __syncwarp();
@@ -281,9 +301,9 @@ force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict
 
 template <int ET, bool J2, int MODE>
 int force_go(exfem_block_s* b, const double* u, const double* st_old, double* st_new, double* fe, double* S,
-             double* mises, double* peeq, cudaStream_t s) {
+             double* mises, double* peeq, cudaStream_t s, const uint8_t* nf = nullptr, const int* skip = nullptr) {
   constexpr int NW = 4;
-  using SM = ForceSmem<ET, J2>;
+  using SM = ForceSmem<ET, J2 && MODE != FORCE_PRODUCT>;
   constexpr size_t smem = NW * sizeof(SM);
   constexpr int64_t per = NW * SM::EPW;
   // bulk copies need 16-byte boundaries: elements' states and forces are multiples of
@@ -292,7 +312,7 @@ int force_go(exfem_block_s* b, const double* u, const double* st_old, double* st
                    ((uintptr_t)fe % 16 == 0 ? BULK_FE : 0);
   force_kernel<ET, J2, MODE, NW><<<(unsigned)((b->ne + per - 1) / per), 32 * NW, smem, s>>>(
       b->ne, b->X.p, b->conn.p, u, b->scale.p, st_old, st_new, fe, b->tan64.p, b->tan32.p, S, mises, peeq, b->mat,
-      b->lam_e.p, b->mu_e.p, b->order_dev.p, b->tile == 128 ? 7 : 8, bulk, b->dev_err.p);
+      b->lam_e.p, b->mu_e.p, b->order_dev.p, b->tile == 128 ? 7 : 8, bulk, b->dev_err.p, nf, skip);
   EX_LAUNCH_CHECK();
   return EXFEM_OK;
 }
@@ -317,6 +337,19 @@ int launch_force(exfem_block_s* b, int mode, const double* u, const double* st_o
   if (b->ne == 0) return EXFEM_OK;
   return b->etype == EXFEM_C3D8 ? force_et<EXFEM_C3D8>(b, mode, u, st_old, st_new, fe, S, mises, peeq, s)
                                 : force_et<EXFEM_C3D10>(b, mode, u, st_old, st_new, fe, S, mises, peeq, s);
+}
+
+// element vectors fe (ne, nnode, 3) of the FP64 tangent product K (free v): the force
+// kernel on v with the linear stress, elastic or of the stored tangent data
+int launch_product_elements(exfem_block_s* b, const double* v, double* fe, bool bc, const int* skip, cudaStream_t s) {
+  if (b->ne == 0) return EXFEM_OK;
+  const uint8_t* nf = bc ? b->node_fixed.p : nullptr;
+  const bool j2 = b->mat.kind == EXFEM_J2;
+#define EXF_GO(ET, J2) \
+  force_go<ET, J2, FORCE_PRODUCT>(b, v, nullptr, nullptr, fe, nullptr, nullptr, nullptr, s, nf, skip)
+  if (b->etype == EXFEM_C3D8) return j2 ? EXF_GO(EXFEM_C3D8, true) : EXF_GO(EXFEM_C3D8, false);
+  return j2 ? EXF_GO(EXFEM_C3D10, true) : EXF_GO(EXFEM_C3D10, false);
+#undef EXF_GO
 }
 
 }  // namespace exfem

@@ -39,7 +39,8 @@ struct NodeSmem {
 
 // Gather of X and u (u may be NULL: zeros) at the nodes of the warp's elements.
 // `eid`: this lane's element; `elem(el)`: the warp's el-th element, called by all lanes;
-// `cnt`: elements of this warp.  The caller synchronises the warp afterwards.
+// `cnt`: elements of this warp; `nf` (or NULL): per node, the components of u taken as
+// zero (bits).  The caller synchronises the warp afterwards.
 //
 // C3D8: a lane loads one of its element's eight nodes and a Walsh-Hadamard transform
 // over the element's lanes turns the corner values into the modal ones (corner signs
@@ -48,17 +49,19 @@ struct NodeSmem {
 template <int ET, bool U, class Elem>
 __device__ __forceinline__ void gather_nodes(NodeSmem<ET, U>& nd, const double* __restrict__ X,
                                              const int32_t* __restrict__ conn, const double* __restrict__ u,
-                                             int64_t eid, int cnt, Elem elem) {
+                                             const uint8_t* __restrict__ nf, int64_t eid, int cnt, Elem elem) {
   constexpr int W = NodeSmem<ET, U>::W, EPW = NodeSmem<ET, U>::EPW, ES = NodeSmem<ET, U>::ES;
   const int lane = threadIdx.x & 31;
   if constexpr (ET == EXFEM_C3D8) {
     const int j = lane & 7, a = j ^ ((j >> 1) & 1);  // bits of j: the corner lies on the + side of each axis
-    const int64_t n3 = 3 * (int64_t)conn[eid * 8 + a];
+    const int32_t node = conn[eid * 8 + a];
+    const int64_t n3 = 3 * (int64_t)node;
+    const unsigned off = U && nf ? nf[node] : 0u;
     double v[W];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       v[c] = X[n3 + c];
-      if constexpr (U) v[3 + c] = u ? u[n3 + c] : 0.0;
+      if constexpr (U) v[3 + c] = u && !((off >> c) & 1u) ? u[n3 + c] : 0.0;
     }
     // relative to the first node: the sums below then carry no rounding of the
     // distance from the origin
@@ -80,11 +83,13 @@ __device__ __forceinline__ void gather_nodes(NodeSmem<ET, U>& nd, const double* 
       const int k = k0 + lane, el = k / NN < EPW ? k / NN : EPW - 1, a = k - el * NN;
       const int64_t e = elem(el);
       if (k < cnt * NN) {
-        const int64_t n3 = 3 * (int64_t)conn[e * NN + a];
+        const int32_t node = conn[e * NN + a];
+        const int64_t n3 = 3 * (int64_t)node;
+        const unsigned off = U && nf ? nf[node] : 0u;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           nd.v[el * ES + a * W + c] = X[n3 + c];
-          if constexpr (U) nd.v[el * ES + a * W + 3 + c] = u ? u[n3 + c] : 0.0;
+          if constexpr (U) nd.v[el * ES + a * W + 3 + c] = u && !((off >> c) & 1u) ? u[n3 + c] : 0.0;
         }
       }
     }

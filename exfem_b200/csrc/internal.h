@@ -67,11 +67,12 @@ struct exfem_block_s {
   // generations: tangent data and boundary-condition buffers (solvers compare)
   uint64_t tan_gen = 0, bc_gen = 0;
   // scratch
-  exfem::DevBuf<double> ys;           // (ne*nnode*3) element vectors for gather assembly
+  exfem::DevBuf<double> ys;           // (ne*nnode*3) element vectors for gather assembly; then those of the FP64 products
   exfem::DevBuf<double> mp_work;      // multi-case Jacobi PCG: inverse diagonal, R, P, Q, partial sums, scalars
   exfem::DevBuf<double> ys_m64;       // (ne*nnode*3*nrhs) element rows of the FP64 multi-right-hand-side product
   exfem::DevBuf<float> ys_tc;         // (ne*nnode*3*nrhs) element rows of the tensor-core stored-Ke product
   int64_t ndof() const { return 3 * nn; }
+  double* ys_product() const { return ys.p + ne * nnode * 3; }  // where product_by_points(etype, ne)
 };
 
 namespace exfem {
@@ -87,9 +88,10 @@ struct Csr64 {  // device CSR, FP64 values and an FP32 copy
   DevBuf<int64_t> rmap, cshift;
 };
 
-// element kernels (element_ops.cu)
+// element kernels (force.cu, stiffness.cu, element_ops.cu)
 int launch_force(exfem_block_s* b, int mode, const double* u, const double* st_old, double* st_new,
                  double* fe, double* S, double* mises, double* peeq, cudaStream_t s);
+int launch_product_elements(exfem_block_s* b, const double* v, double* fe, bool bc, const int* skip, cudaStream_t s);
 int launch_gather_assemble(exfem_block_s* b, const double* ys, double* f, const double* v_opa,
                            const int* skip, cudaStream_t s);
 int build_geometry(exfem_block_s* b);
@@ -104,6 +106,7 @@ int launch_geo_stiffness(exfem_block_s* b, const double* S, double* Kg, cudaStre
 template <class T>
 int launch_mf_matvec(exfem_block_s* b, const T* v, T* y, const int* skip, cudaStream_t s, bool bc = true);
 int launch_mf_diagonal(exfem_block_s* b, double* diag, cudaStream_t s);
+bool product_by_points(int etype, int64_t ne);  // FP64 products through element vectors
 // bounded device waits: read and clear a block's wait-failure flag (capi.cu); a
 // kernel whose only wait can never complete (matfree.cu)
 int block_wait_status(exfem_block_s* b, cudaStream_t s);
@@ -122,6 +125,6 @@ template <class VT>
 int launch_gather_multi(exfem_block_s* b, const VT* ys, const VT* V, VT* Y, int nrhs, bool bc, cudaStream_t s);
 
 // reductions and vector kernels (krylov.cu)
-enum ModeForce { FORCE_FULL = 0, FORCE_TANGENT = 1, FORCE_STRESS = 2 };
+enum ModeForce { FORCE_FULL = 0, FORCE_TANGENT = 1, FORCE_STRESS = 2, FORCE_PRODUCT = 3 };
 
 }  // namespace exfem

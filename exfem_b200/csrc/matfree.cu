@@ -791,6 +791,15 @@ static int mf_dispatch(exfem_block_s* b, const T* geo, const T* tan, const int32
   return mf_tile<T, ET, false, false>(b, geo, tan, tpack, v, y, part, skip, s);
 }
 
+// FP64 products: one lane per Gauss point writing element vectors (force.cu) and the
+// gather assembly, or the tiles above.  The points' form recomputes the geometry at
+// each point, but a mesh spreads over the chip from a few elements on and its code is
+// short (the tiles' unrolled FP64 element takes a warp about 25 us however small the
+// mesh); the tiles do less arithmetic per element.  B200, points / tiles: C3D8 320
+// elements 5.8 / 29 us, 40,000 21 / 42, 126,000 56 / 57, 320,000 145 / 94; C3D10 900
+// elements 8.6 / 34, 113,724 38 / 70, 384,000 135 / 136, 1,053,696 380 / 343 (J2 alike).
+bool product_by_points(int etype, int64_t ne) { return ne <= (etype == EXFEM_C3D8 ? 120000 : 350000); }
+
 template <class T>
 int launch_mf_matvec(exfem_block_s* b, const T* v, T* y, const int* skip, cudaStream_t s, bool bc) {
   const int64_t ndof = b->ndof();
@@ -798,6 +807,13 @@ int launch_mf_matvec(exfem_block_s* b, const T* v, T* y, const int* skip, cudaSt
   if (b->etype == EXFEM_C3D10 && !b->affine) {
     set_error("matrix-free C3D10 needs straight-edged elements (mid-nodes at edge midpoints)");
     return EXFEM_ERR_UNSUPPORTED;
+  }
+  if constexpr (sizeof(T) == 8) {
+    if (product_by_points(b->etype, b->ne)) {
+      const int st = launch_product_elements(b, v, b->ys_product(), bc, skip, s);
+      if (st) return st;
+      return launch_gather_assemble(b, b->ys_product(), y, bc ? v : nullptr, skip, s);
+    }
   }
   T* part = reinterpret_cast<T*>(b->partial.p);
   if (b->ne) {
