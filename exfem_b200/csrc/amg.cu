@@ -97,13 +97,20 @@ static int spmv_lanes(const Csr64& A, const T* val, const T* x, T* y, const T* b
 template <class T, int N, int A>
 __device__ __forceinline__ void load_regs(const T* __restrict__ p, T (&o)[N]) {
   constexpr int BYTES = N * (int)sizeof(T);
-  if constexpr (A % 16 == 0 && BYTES % 16 == 0) {
+  if constexpr (sizeof(T) == 8 && A % 16 == 0 && N % 2 == 0) {
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+      const double2 v = __ldg(reinterpret_cast<const double2*>(p) + i);
+      o[2 * i] = v.x;
+      o[2 * i + 1] = v.y;
+    }
+  } else if constexpr (sizeof(T) == 4 && A % 16 == 0 && BYTES % 16 == 0) {
 #pragma unroll
     for (int i = 0; i < BYTES / 16; ++i) {
       const float4 v = __ldg(reinterpret_cast<const float4*>(p) + i);
       memcpy(reinterpret_cast<char*>(o) + 16 * i, &v, 16);
     }
-  } else if constexpr (A % 8 == 0 && BYTES % 8 == 0) {
+  } else if constexpr (sizeof(T) == 4 && A % 8 == 0 && BYTES % 8 == 0) {
 #pragma unroll
     for (int i = 0; i < BYTES / 8; ++i) {
       const float2 v = __ldg(reinterpret_cast<const float2*>(p) + i);
@@ -121,76 +128,133 @@ constexpr int stride_align() {
   return (N * (int)sizeof(T)) % 16 == 0 ? 16 : (N * (int)sizeof(T)) % 8 == 0 ? 8 : 4;
 }
 
-// Block-sparse product with the same fused modes as spmv_kernel: L lanes per block
-// row stride over its blocks (consecutive blocks are contiguous in memory, so a
-// group's loads coalesce), each lane keeps the R row sums of its blocks, and the
-// group reduces them in a fixed order; lane 0 finishes the R rows.
+// Block-sparse product with the same fused modes as spmv_kernel: L lanes per block row
+// (up to a whole thread block for the long rows of a restriction) take its blocks in
+// turn, U of them requested before the first is used; the R row sums are reduced over
+// the lanes in a fixed order, and lane i finishes row i from operands it requested at
+// the start.
+//
+// Bound by latency on the coarser levels (row pointer -> column -> x -> epilogue), so
+// lanes are chosen for about two blocks each.  B200, FP32, a 480,975-row mesh level over
+// 6,390 and 162 rows, measured inside the solver's graph: mesh restriction 39 -> 15 us,
+// products of the 6,390-row level 10-13 -> 4 us, its restriction 19 -> 7 us against at
+// most 32 lanes, one block in flight per lane and the whole epilogue on lane 0.
 template <class T, int R, int C, int L, int MODE>
 __global__ void __launch_bounds__(256)
 bsr_kernel(int64_t nb, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx, const T* __restrict__ val,
            const T* __restrict__ x, T* __restrict__ y, const T* __restrict__ b, const T* __restrict__ dinv,
            T* __restrict__ d2, T* __restrict__ xo, T c1, T c2, const int* __restrict__ skip) {
   if (skip && *skip) return;
-  constexpr int GPW = 32 / L;
-  const int lane = threadIdx.x & (L - 1);
-  const int grp = (threadIdx.x & 31) / L;
-  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t base = warp * GPW; base < nb; base += nwarps * GPW) {
-    const int64_t br = base + grp;
+  constexpr int RPB = 256 / L;                        // block rows per thread block
+  constexpr int WL = L < 32 ? L : 32;                 // lanes of a row within a warp
+  constexpr int WR = L > 32 ? L / 32 : 1;             // warps per row
+  constexpr int BB = R * C * (int)sizeof(T);
+  constexpr int U = BB >= 288 ? 1 : (BB >= 144 ? 2 : 4);
+  static_assert(WL >= R || L < 32, "rows of a wide group are finished by one lane each");
+  constexpr int PER = (R + WL - 1) / WL;              // rows a lane finishes
+  __shared__ T part[L > 32 ? 8 : 1][R];
+  const int lane = threadIdx.x % L, wl = threadIdx.x & (WL - 1);
+  for (int64_t base = (int64_t)blockIdx.x * RPB; base < nb; base += (int64_t)gridDim.x * RPB) {
+    const int64_t br = base + threadIdx.x / L;
+    const bool in = br < nb;
+    // this lane's rows: their epilogue operands
+    T e0[PER], e1[PER], e2[PER], e3[PER];
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+      const int i = wl + p * WL;
+      e0[p] = e1[p] = e2[p] = e3[p] = T(0);
+      if (in && lane < WL && i < R) {
+        const int64_t row = br * R + i;
+        if (MODE == SP_ADD) e0[p] = y[row];
+        if (MODE == SP_RES) e0[p] = b[row];
+        if (MODE == SP_RESINIT) { e0[p] = b[row]; e1[p] = dinv[row]; }
+        if (MODE == SP_CHEB || MODE == SP_CHEBLAST) {
+          e0[p] = y[row];
+          e1[p] = dinv[row];
+          e2[p] = x[row];  // x is the direction d
+          e3[p] = xo[row];
+        }
+      }
+    }
     T acc[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) acc[i] = T(0);
-    if (br < nb) {
+    if (in) {
       const int64_t k1 = ptr[br + 1];
-      for (int64_t k = ptr[br] + lane; k < k1; k += L) {
-        T v[R * C], xv[C];
-        load_regs<T, R * C, stride_align<T, R * C>()>(val + k * (R * C), v);
-        load_regs<T, C, stride_align<T, C>()>(x + (int64_t)idx[k] * C, xv);
-        if constexpr (MODE == SP_SETDIFF) {
-          T bv[C];
-          load_regs<T, C, stride_align<T, C>()>(b + (int64_t)idx[k] * C, bv);
+      for (int64_t k0 = ptr[br] + lane; k0 < k1; k0 += U * L) {
+        int32_t col[U];
+        T v[U][R * C], xv[U][C];
 #pragma unroll
-          for (int j = 0; j < C; ++j) xv[j] = bv[j] - xv[j];
+        for (int u = 0; u < U; ++u) {
+          const int64_t k = k0 + u * L;
+          col[u] = k < k1 ? idx[k] : -1;
+          if (k < k1) load_regs<T, R * C, stride_align<T, R * C>()>(val + k * (R * C), v[u]);
         }
 #pragma unroll
-        for (int i = 0; i < R; ++i)
+        for (int u = 0; u < U; ++u)
+          if (col[u] >= 0) {
+            load_regs<T, C, stride_align<T, C>()>(x + (int64_t)col[u] * C, xv[u]);
+            if constexpr (MODE == SP_SETDIFF) {
+              T bv[C];
+              load_regs<T, C, stride_align<T, C>()>(b + (int64_t)col[u] * C, bv);
 #pragma unroll
-          for (int j = 0; j < C; ++j) acc[i] += v[i * C + j] * xv[j];
+              for (int j = 0; j < C; ++j) xv[u][j] = bv[j] - xv[u][j];
+            }
+          }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (col[u] >= 0)
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+#pragma unroll
+              for (int j = 0; j < C; ++j) acc[i] += v[u][i * C + j] * xv[u][j];
       }
     }
 #pragma unroll
     for (int i = 0; i < R; ++i)
 #pragma unroll
-      for (int o = L / 2; o > 0; o >>= 1) acc[i] += __shfl_down_sync(0xffffffffu, acc[i], o, L);
-    if (br < nb && lane == 0) {
+      for (int o = WL / 2; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+    if constexpr (L > 32) {  // the row's warps in order
+      __syncthreads();
+      if (wl == 0)
 #pragma unroll
-      for (int i = 0; i < R; ++i) {
-        const int64_t row = br * R + i;
-        const T sv = acc[i];
-        if (MODE == SP_SET) {
-          y[row] = sv;
-        } else if (MODE == SP_ADD) {
-          y[row] += sv;
-        } else if (MODE == SP_RES) {
-          y[row] = b[row] - sv;
-        } else if (MODE == SP_RESINIT) {
-          const T r = dinv[row] * (b[row] - sv);
+        for (int i = 0; i < R; ++i) part[threadIdx.x >> 5][i] = acc[i];
+      __syncthreads();
+      if (lane < WL) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          acc[i] = T(0);
+#pragma unroll
+          for (int w = 0; w < WR; ++w) acc[i] += part[(threadIdx.x >> 5) + w][i];
+        }
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+      const int i = wl + p * WL;
+      if (!(in && lane < WL && i < R)) continue;
+      T sv = acc[0];
+#pragma unroll
+      for (int r = 1; r < R; ++r) sv = i == r ? acc[r] : sv;
+      const int64_t row = br * R + i;
+      if (MODE == SP_SET || MODE == SP_SETDIFF) {
+        y[row] = sv;
+      } else if (MODE == SP_ADD) {
+        y[row] = e0[p] + sv;
+      } else if (MODE == SP_RES) {
+        y[row] = e0[p] - sv;
+      } else if (MODE == SP_RESINIT) {
+        const T r = e1[p] * (e0[p] - sv);
+        y[row] = r;
+        d2[row] = r * c1;
+      } else {
+        const T d = e2[p], r = e0[p] - e1[p] * sv, dn = c1 * d + c2 * r;
+        if (MODE == SP_CHEB) {
+          xo[row] = e3[p] + d;
           y[row] = r;
-          d2[row] = r * c1;
-        } else if (MODE == SP_CHEB) {  // x is the direction d
-          const T d = x[row];
-          xo[row] += d;
-          const T r = y[row] - dinv[row] * sv;
-          y[row] = r;
-          d2[row] = c1 * d + c2 * r;
-        } else if (MODE == SP_CHEBLAST) {
-          const T d = x[row];
-          const T r = y[row] - dinv[row] * sv;
-          const T dn = c1 * d + c2 * r;
-          xo[row] = (xo[row] + d) + dn;
-        } else {  // SP_SETDIFF
-          y[row] = sv;
+          d2[row] = dn;
+        } else {  // SP_CHEBLAST
+          xo[row] = (e3[p] + d) + dn;
         }
       }
     }
@@ -207,14 +271,20 @@ static int bsr_launch(const Bsr& M, const T* val, const T* x, T* y, const T* b, 
     return EXFEM_ERR_ARG;
   }
   const double avg = M.nb ? (double)M.nnzb / (double)M.nb : 0.0;
-  const int threads = 256;
-  // one group of L lanes per block row: 32 / L block rows per warp
-#define EXF_BSR(L) bsr_kernel<T, R, C, L, MODE><<<grid_for((size_t)((M.nb + 32 / L - 1) / (32 / L)) * 32, threads, 148u * 24u), threads, 0, s>>>(M.nb, M.ptr.p, M.idx.p, val, x, y, b, dinv, d2, xo, c1, c2, skip)
-  if (avg <= 2) EXF_BSR(1);
-  else if (avg <= 6) EXF_BSR(4);
+  // about two blocks per lane; rows of up to four blocks take single lanes once four
+  // lanes a row would exceed the threads the chip holds (148 x 2,048): their blocks then
+  // stream by (FP64 prolongation to 160,325 rows: 50 us less an iteration; to
+  // 44,541 rows four lanes are 4 us faster)
+#define EXF_BSR(L)                                                                                                   \
+  bsr_kernel<T, R, C, L, MODE><<<grid_for((size_t)((M.nb + 256 / L - 1) / (256 / L)) * 256, 256, 148u * 24u), 256, 0, \
+                                 s>>>(M.nb, M.ptr.p, M.idx.p, val, x, y, b, dinv, d2, xo, c1, c2, skip)
+  if (avg <= 2 || (avg <= 4 && M.nb > 148 * 512)) EXF_BSR(1);
+  else if (avg <= 8) EXF_BSR(4);
   else if (avg <= 16) EXF_BSR(8);
-  else if (avg <= 40) EXF_BSR(16);
-  else EXF_BSR(32);
+  else if (avg <= 32) EXF_BSR(16);
+  else if (avg <= 96) EXF_BSR(32);
+  else if (avg <= 256) EXF_BSR(64);
+  else EXF_BSR(256);
 #undef EXF_BSR
   return EXFEM_OK;
 }
