@@ -15,6 +15,7 @@
 // element kernel and the vector updates through small elementwise kernels.
 #include <array>
 #include <mutex>
+#include <type_traits>
 
 #include "internal.h"
 #include "solver.h"
@@ -93,34 +94,40 @@ static int spmv_lanes(const Csr64& A, const T* val, const T* x, T* y, const T* b
 }
 
 // N values of T from p into registers with the widest loads that p's alignment A
-// (bytes, a multiple of 4) allows: 16-byte, 8-byte or single loads.
-template <class T, int N, int A>
-__device__ __forceinline__ void load_regs(const T* __restrict__ p, T (&o)[N]) {
-  constexpr int BYTES = N * (int)sizeof(T);
-  if constexpr (sizeof(T) == 8 && A % 16 == 0 && N % 2 == 0) {
+// (bytes, a multiple of 4) allows: 16-byte, 8-byte or single loads.  load_regs: of data
+// constant over the launch; load_vec: of vectors the kernel ahead may have written.
+template <bool CONST, class V>
+__device__ __forceinline__ V load_one(const V* p) {
+  if constexpr (CONST) return __ldg(p);
+  else return *p;
+}
+template <bool CONST, class T, int N, int A>
+__device__ __forceinline__ void load_n(const T* p, T (&o)[N]) {
+  constexpr int W = A % 16 == 0 && (N * sizeof(T)) % 16 == 0 ? 16 / (int)sizeof(T)
+                    : A % 8 == 0 && (N * sizeof(T)) % 8 == 0 ? 8 / (int)sizeof(T)
+                                                             : 1;
 #pragma unroll
-    for (int i = 0; i < N / 2; ++i) {
-      const double2 v = __ldg(reinterpret_cast<const double2*>(p) + i);
+  for (int i = 0; i < N / W; ++i) {
+    if constexpr (W == 4) {
+      const float4 v = load_one<CONST>(reinterpret_cast<const float4*>(p) + i);
+      o[4 * i] = v.x;
+      o[4 * i + 1] = v.y;
+      o[4 * i + 2] = v.z;
+      o[4 * i + 3] = v.w;
+    } else if constexpr (W == 2) {
+      using V = std::conditional_t<sizeof(T) == 8, double2, float2>;
+      const V v = load_one<CONST>(reinterpret_cast<const V*>(p) + i);
       o[2 * i] = v.x;
       o[2 * i + 1] = v.y;
+    } else {
+      o[i] = load_one<CONST>(p + i);
     }
-  } else if constexpr (sizeof(T) == 4 && A % 16 == 0 && BYTES % 16 == 0) {
-#pragma unroll
-    for (int i = 0; i < BYTES / 16; ++i) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(p) + i);
-      memcpy(reinterpret_cast<char*>(o) + 16 * i, &v, 16);
-    }
-  } else if constexpr (sizeof(T) == 4 && A % 8 == 0 && BYTES % 8 == 0) {
-#pragma unroll
-    for (int i = 0; i < BYTES / 8; ++i) {
-      const float2 v = __ldg(reinterpret_cast<const float2*>(p) + i);
-      memcpy(reinterpret_cast<char*>(o) + 8 * i, &v, 8);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < N; ++i) o[i] = __ldg(p + i);
   }
 }
+template <class T, int N, int A>
+__device__ __forceinline__ void load_regs(const T* p, T (&o)[N]) { load_n<true, T, N, A>(p, o); }
+template <class T, int N, int A>
+__device__ __forceinline__ void load_vec(const T* p, T (&o)[N]) { load_n<false, T, N, A>(p, o); }
 
 // alignment in bytes of element k * n of a 256-byte aligned array of T
 template <class T, int N>
@@ -142,9 +149,7 @@ constexpr int stride_align() {
 template <class T, int R, int C, int L, int MODE>
 __global__ void __launch_bounds__(256)
 bsr_kernel(int64_t nb, const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx, const T* __restrict__ val,
-           const T* __restrict__ x, T* __restrict__ y, const T* __restrict__ b, const T* __restrict__ dinv,
-           T* __restrict__ d2, T* __restrict__ xo, T c1, T c2, const int* __restrict__ skip) {
-  if (skip && *skip) return;
+           const T* x, T* y, const T* b, const T* dinv, T* d2, T* xo, T c1, T c2, const int* skip) {
   constexpr int RPB = 256 / L;                        // block rows per thread block
   constexpr int WL = L < 32 ? L : 32;                 // lanes of a row within a warp
   constexpr int WR = L > 32 ? L / 32 : 1;             // warps per row
@@ -154,9 +159,29 @@ bsr_kernel(int64_t nb, const int64_t* __restrict__ ptr, const int32_t* __restric
   constexpr int PER = (R + WL - 1) / WL;              // rows a lane finishes
   __shared__ T part[L > 32 ? 8 : 1][R];
   const int lane = threadIdx.x % L, wl = threadIdx.x & (WL - 1);
+  bool waited = false;
   for (int64_t base = (int64_t)blockIdx.x * RPB; base < nb; base += (int64_t)gridDim.x * RPB) {
     const int64_t br = base + threadIdx.x / L;
     const bool in = br < nb;
+    // the matrix is constant: the first blocks are requested before the wait
+    int64_t k0 = in ? ptr[br] + lane : 0;
+    const int64_t k1 = in ? ptr[br + 1] : 0;
+    int32_t col[U];
+    T v[U][R * C];
+    auto blocks = [&]() {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t k = k0 + u * L;
+        col[u] = k < k1 ? idx[k] : -1;
+        if (k < k1) load_regs<T, R * C, stride_align<T, R * C>()>(val + k * (R * C), v[u]);
+      }
+    };
+    blocks();
+    if (!waited) {
+      chain_wait();
+      waited = true;
+      if (skip && *skip) return;
+    }
     // this lane's rows: their epilogue operands
     T e0[PER], e1[PER], e2[PER], e3[PER];
 #pragma unroll
@@ -179,36 +204,28 @@ bsr_kernel(int64_t nb, const int64_t* __restrict__ ptr, const int32_t* __restric
     T acc[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) acc[i] = T(0);
-    if (in) {
-      const int64_t k1 = ptr[br + 1];
-      for (int64_t k0 = ptr[br] + lane; k0 < k1; k0 += U * L) {
-        int32_t col[U];
-        T v[U][R * C], xv[U][C];
+    while (k0 < k1) {
+      T xv[U][C];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int64_t k = k0 + u * L;
-          col[u] = k < k1 ? idx[k] : -1;
-          if (k < k1) load_regs<T, R * C, stride_align<T, R * C>()>(val + k * (R * C), v[u]);
+      for (int u = 0; u < U; ++u)
+        if (col[u] >= 0) {
+          load_vec<T, C, stride_align<T, C>()>(x + (int64_t)col[u] * C, xv[u]);
+          if constexpr (MODE == SP_SETDIFF) {
+            T bv[C];
+            load_vec<T, C, stride_align<T, C>()>(b + (int64_t)col[u] * C, bv);
+#pragma unroll
+            for (int j = 0; j < C; ++j) xv[u][j] = bv[j] - xv[u][j];
+          }
         }
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (col[u] >= 0) {
-            load_regs<T, C, stride_align<T, C>()>(x + (int64_t)col[u] * C, xv[u]);
-            if constexpr (MODE == SP_SETDIFF) {
-              T bv[C];
-              load_regs<T, C, stride_align<T, C>()>(b + (int64_t)col[u] * C, bv);
+      for (int u = 0; u < U; ++u)
+        if (col[u] >= 0)
 #pragma unroll
-              for (int j = 0; j < C; ++j) xv[u][j] = bv[j] - xv[u][j];
-            }
-          }
+          for (int i = 0; i < R; ++i)
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (col[u] >= 0)
-#pragma unroll
-            for (int i = 0; i < R; ++i)
-#pragma unroll
-              for (int j = 0; j < C; ++j) acc[i] += v[u][i * C + j] * xv[u][j];
-      }
+            for (int j = 0; j < C; ++j) acc[i] += v[u][i * C + j] * xv[u][j];
+      k0 += U * L;
+      if (k0 < k1) blocks();
     }
 #pragma unroll
     for (int i = 0; i < R; ++i)
@@ -276,8 +293,9 @@ static int bsr_launch(const Bsr& M, const T* val, const T* x, T* y, const T* b, 
   // stream by (FP64 prolongation to 160,325 rows: 50 us less an iteration; to
   // 44,541 rows four lanes are 4 us faster)
 #define EXF_BSR(L)                                                                                                   \
-  bsr_kernel<T, R, C, L, MODE><<<grid_for((size_t)((M.nb + 256 / L - 1) / (256 / L)) * 256, 256, 148u * 24u), 256, 0, \
-                                 s>>>(M.nb, M.ptr.p, M.idx.p, val, x, y, b, dinv, d2, xo, c1, c2, skip)
+  launch_chained(bsr_kernel<T, R, C, L, MODE>,                                                                        \
+                 grid_for((size_t)((M.nb + 256 / L - 1) / (256 / L)) * 256, 256, 148u * 24u), 256, 0, s, M.nb, M.ptr.p, \
+                 M.idx.p, val, x, y, b, dinv, d2, xo, c1, c2, skip)
   if (avg <= 2 || (avg <= 4 && M.nb > 148 * 512)) EXF_BSR(1);
   else if (avg <= 8) EXF_BSR(4);
   else if (avg <= 16) EXF_BSR(8);
@@ -316,9 +334,9 @@ template <> const float* csr_vals<float>(const Csr64& A) { return A.v32.p; }
 
 // ---------------------------------------------------------------- elementwise kernels
 template <class T>
-__global__ void cheb_init0_kernel(int64_t n, const T* __restrict__ b, const T* __restrict__ dinv,
-                                  T* __restrict__ x, T* __restrict__ r, T* __restrict__ d, T ith,
-                                  const int* __restrict__ skip, const T* __restrict__ rith = nullptr) {
+__global__ void cheb_init0_kernel(int64_t n, const T* b, const T* dinv, T* x, T* r, T* d, T ith,
+                                  const int* skip, const T* __restrict__ rith) {
+  chain_wait();
   if (skip && *skip) return;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const T ri = dinv[i] * b[i];
@@ -329,10 +347,10 @@ __global__ void cheb_init0_kernel(int64_t n, const T* __restrict__ b, const T* _
 }
 
 template <class T>
-__global__ void cheb_update_kernel(int64_t n, T* __restrict__ x, const T* __restrict__ d, T* __restrict__ r,
-                                   const T* __restrict__ Ad, const T* __restrict__ dinv, T* __restrict__ d2,
-                                   T c1, T c2, const int* __restrict__ skip, const T* __restrict__ rc1 = nullptr,
-                                   const T* __restrict__ rc2 = nullptr, int last = 0) {
+__global__ void cheb_update_kernel(int64_t n, T* x, const T* d, T* r, const T* Ad,
+                                   const T* dinv, T* d2, T c1, T c2, const int* skip,
+                                   const T* __restrict__ rc1, const T* __restrict__ rc2, int last) {
+  chain_wait();
   if (skip && *skip) return;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const T di = d[i];
@@ -349,9 +367,9 @@ __global__ void cheb_update_kernel(int64_t n, T* __restrict__ x, const T* __rest
 }
 
 template <class T>
-__global__ void resinit_kernel(int64_t n, const T* __restrict__ b, const T* __restrict__ Ax,
-                               const T* __restrict__ dinv, T* __restrict__ r, T* __restrict__ d, T ith,
-                               const int* __restrict__ skip, const T* __restrict__ rith = nullptr) {
+__global__ void resinit_kernel(int64_t n, const T* b, const T* Ax, const T* dinv, T* r, T* d, T ith,
+                               const int* skip, const T* __restrict__ rith) {
+  chain_wait();
   if (skip && *skip) return;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const T ri = dinv[i] * (b[i] - Ax[i]);
@@ -376,8 +394,8 @@ __global__ void add_kernel(int64_t n, const T* __restrict__ d, T* __restrict__ x
 
 // x = Ainv * b, FP64 arithmetic, one warp per row
 template <class T>
-__global__ void coarse_kernel(int64_t nc, const double* __restrict__ Ainv, const T* __restrict__ b,
-                              T* __restrict__ x, const int* __restrict__ skip) {
+__global__ void coarse_kernel(int64_t nc, const double* __restrict__ Ainv, const T* b, T* x, const int* skip) {
+  chain_wait();
   if (skip && *skip) return;
   const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -451,7 +469,8 @@ static int coarse_solve(exfem_amg_s* h, const T* b, T* x, const int* skip, cudaS
     EX_LAUNCH_CHECK();
     return EXFEM_OK;
   }
-  coarse_kernel<T><<<(unsigned)((h->nc * 32 + threads - 1) / threads), threads, 0, s>>>(h->nc, h->Ainv.p, b, x, skip);
+  launch_chained(coarse_kernel<T>, (unsigned)((h->nc * 32 + threads - 1) / threads), threads, 0, s, h->nc, h->Ainv.p, b,
+                 x, skip);
   EX_LAUNCH_CHECK();
   return EXFEM_OK;
 }
@@ -503,9 +522,8 @@ static int vcycle_level(exfem_amg_s* h, size_t l, const T* b, T* x, const Level0
       const bool last = fused_last && j == h->degree - 1;
       if (mf) {
         if ((st = op0->apply(op0->ctx, d, t, skip, s))) return st;
-        cheb_update_kernel<T><<<eg, 256, 0, s>>>(n, x, d, r, t, dinv, d2, (T)ca[j], (T)cb[j], skip,
-                                                 rc ? rc + 2 * j : nullptr, rc ? rc + 2 * j + 1 : nullptr,
-                                                 last ? 1 : 0);
+        launch_chained(cheb_update_kernel<T>, eg, 256, 0, s, n, x, d, r, t, dinv, d2, (T)ca[j], (T)cb[j], skip,
+                       rc ? rc + 2 * j : nullptr, rc ? rc + 2 * j + 1 : nullptr, last ? 1 : 0);
         EX_LAUNCH_CHECK();
       } else {
         if (useA) {
@@ -529,7 +547,7 @@ static int vcycle_level(exfem_amg_s* h, size_t l, const T* b, T* x, const Level0
     return EXFEM_OK;
   };
   // pre-smoothing from x = 0
-  cheb_init0_kernel<T><<<eg, 256, 0, s>>>(n, b, dinv, x, r, d, ith, skip, rc ? rc + 4 : nullptr);
+  launch_chained(cheb_init0_kernel<T>, eg, 256, 0, s, n, b, dinv, x, r, d, ith, skip, rc ? rc + 4 : nullptr);
   EX_LAUNCH_CHECK();
   if ((st = smooth_steps())) return st;
   // residual and restriction
@@ -576,7 +594,7 @@ static int vcycle_level(exfem_amg_s* h, size_t l, const T* b, T* x, const Level0
   // post-smoothing from the corrected x
   if (mf) {
     if ((st = op0->apply(op0->ctx, x, t, skip, s))) return st;
-    resinit_kernel<T><<<eg, 256, 0, s>>>(n, b, t, dinv, r, d, ith, skip, rc ? rc + 4 : nullptr);
+    launch_chained(resinit_kernel<T>, eg, 256, 0, s, n, b, t, dinv, r, d, ith, skip, rc ? rc + 4 : nullptr);
     EX_LAUNCH_CHECK();
   } else {
     if (useA) {
@@ -896,7 +914,7 @@ static int vcycle_level_noalloc(exfem_amg_s* h, size_t l, const T* b, T* x, cons
       if (mf) {
         if ((st = op0->apply(op0->ctx, d, t, nullptr, s))) return st;
         cheb_update_kernel<T><<<eg, 256, 0, s>>>(n, x, d, r, t, dinv, d2, (T)ca[j], (T)cb[j], nullptr,
-                                                 rc ? rc + 2 * j : nullptr, rc ? rc + 2 * j + 1 : nullptr);
+                                                 rc ? rc + 2 * j : nullptr, rc ? rc + 2 * j + 1 : nullptr, 0);
         EX_LAUNCH_CHECK();
       } else {
         if ((st = spmv_lanes<T, SP_CHEB>(L.A, vals, d, r, nullptr, dinv, d2, x, (T)ca[j], (T)cb[j], nullptr, s,

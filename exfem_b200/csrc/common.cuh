@@ -120,6 +120,35 @@ inline unsigned grid_for(size_t n, int block, unsigned cap = 148u * 16u) {
   return (unsigned)g;
 }
 
+// ---------------------------------------------------------------- programmatic launches
+// The kernels of a solve form one chain of short launches.  Those started with
+// launch_chained may begin before the kernel ahead of them in the stream has finished:
+// they load what no launch of the chain writes (mesh maps, matrices) first, call
+// chain_wait() — which returns once that kernel is complete and its writes are visible —
+// before any other global access, and let their own successor start.  Every kernel
+// launched this way calls chain_wait() in every block, so completion carries along the
+// chain.  What is read or written after the wait must not be declared __restrict__: such
+// accesses may be moved ahead of it.
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <class... K, class... A>
+inline void launch_chained(void (*kernel)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A&&... a) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = at;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, kernel, static_cast<K>(a)...);  // errors: EX_LAUNCH_CHECK
+}
+
 // ---------------------------------------------------------------- 3x3 helpers
 // Matrices are row-major T[9]: m[3*i + j].
 template <class T>

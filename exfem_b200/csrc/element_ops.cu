@@ -17,22 +17,26 @@ namespace exfem {
 // for 44,541 nodes of C3D8 and 27 us for 176,715 of C3D10.
 __global__ void __launch_bounds__(256)
 gather_assemble_kernel(int64_t ndof, int vmax, const int32_t* __restrict__ plan, int32_t sentinel,
-                       const double* __restrict__ ys, double* __restrict__ f, const uint8_t* __restrict__ fixed,
-                       const double* __restrict__ v, const int* __restrict__ skip) {
+                       const double* ys, double* f, const uint8_t* __restrict__ fixed, const double* v,
+                       const int* skip) {
   constexpr int K = 8;
-  if (skip && *skip) return;
   const int64_t d = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (d >= ndof) return;
-  const int64_t n = d / 3;
-  const int c = (int)(d - 3 * n);
+  const bool in = d < ndof;
+  const int64_t n = in ? d / 3 : 0;
+  const int c = in ? (int)(d - 3 * n) : 0;
   const int32_t* row = plan + n * vmax;
-  const bool pass = v && fixed && fixed[d];
+  const bool pass = in && v && fixed && fixed[d];
+  int32_t slot[K];  // the plan is constant: its first slots are requested before the wait
+#pragma unroll
+  for (int k = 0; k < K; ++k) slot[k] = k < vmax ? row[k] : sentinel;
+  chain_wait();
+  if (!in || (skip && *skip)) return;
   double s = 0.0;
   for (int k0 = 0; k0 < vmax; k0 += K) {
-    int32_t slot[K];
     double w[K];
+    if (k0 > 0)
 #pragma unroll
-    for (int k = 0; k < K; ++k) slot[k] = k0 + k < vmax ? row[k0 + k] : sentinel;
+      for (int k = 0; k < K; ++k) slot[k] = k0 + k < vmax ? row[k0 + k] : sentinel;
 #pragma unroll
     for (int k = 0; k < K; ++k) w[k] = slot[k] != sentinel ? ys[3 * (int64_t)slot[k] + c] : 0.0;
 #pragma unroll
@@ -47,8 +51,9 @@ int launch_gather_assemble(exfem_block_s* b, const double* ys, double* f, const 
                            const int* skip, cudaStream_t s) {
   if (b->nn == 0) return EXFEM_OK;
   const int threads = 256;
-  gather_assemble_kernel<<<(unsigned)((b->ndof() + threads - 1) / threads), threads, 0, s>>>(
-      b->ndof(), b->vmax, b->plan.p, (int32_t)(b->ne * b->nnode), ys, f, v_opa ? b->fixed.p : nullptr, v_opa, skip);
+  launch_chained(gather_assemble_kernel, (unsigned)((b->ndof() + threads - 1) / threads), threads, 0, s, b->ndof(),
+                 b->vmax, b->plan.p, (int32_t)(b->ne * b->nnode), ys, f,
+                 (const uint8_t*)(v_opa ? b->fixed.p : nullptr), v_opa, skip);
   EX_LAUNCH_CHECK();
   return EXFEM_OK;
 }

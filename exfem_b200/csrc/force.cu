@@ -54,19 +54,22 @@ constexpr int force_warps() {
 template <int ET, bool J2, int MODE, int NW>
 __global__ void __launch_bounds__(32 * NW, force_warps<ET, J2, MODE>() / NW)
 force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict__ conn,
-             const double* __restrict__ u, const double* __restrict__ scale, const double* st_old, double* st_new,
-             double* __restrict__ fe, double* __restrict__ tan64, float* __restrict__ tan32, double* __restrict__ S,
+             const double* u, const double* __restrict__ scale, const double* st_old, double* st_new,
+             double* fe, double* tan64, float* __restrict__ tan32, double* __restrict__ S,
              double* __restrict__ mises, double* __restrict__ peeq, const __grid_constant__ MatDev mat,
              const double* __restrict__ lam_e, const double* __restrict__ mu_e, const int32_t* __restrict__ order,
              int tile_log2, int bulk, int* __restrict__ err, const uint8_t* __restrict__ nf,
-             const int* __restrict__ skip) {
+             const int* skip) {
   using SM = ForceSmem<ET, J2 && MODE != FORCE_PRODUCT>;
   constexpr int NN = SM::NN, NG = SM::NG, ND = SM::ND, EPW = SM::EPW, ST = SM::ST, XS = DnTable<ET>::XS;
   constexpr bool BBAR = SM::BBAR;
   constexpr bool TILED = J2 && MODE != FORCE_STRESS;  // walked in tile order
   constexpr bool PRODUCT = MODE == FORCE_PRODUCT, OUT = MODE == FORCE_FULL || PRODUCT, STATES = J2 && !PRODUCT;
   constexpr int MT = NN > 8 ? 2 : 1, NTC = (3 * EPW + 7) / 8, KS = NG * 3 / 4 + (BBAR ? 1 : 0);
-  if (PRODUCT && skip && *skip) return;
+  if (PRODUCT && skip) {
+    chain_wait();
+    if (*skip) return;
+  }
   __shared__ __align__(16) double tab[NG * XS];
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -102,7 +105,9 @@ force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict
       }
     }
   }
-  gather_nodes<ET, true>(sm.nd, X, conn, u, nf, eid, cnt, elem);
+  gather_nodes<ET, true>(sm.nd, X, conn, u, nf, eid, cnt, elem, [&] {
+    if (PRODUCT && !skip) chain_wait();  // products are chained launches: u is the vector of the one ahead
+  });
   // tile_index(pos, 8 g + k, 8 ngp, tile) for a power of two
   const int64_t tan0 =
       TILED ? (((pos >> tile_log2) * (NG * 8) + g * 8) << tile_log2) + (pos & ((1 << tile_log2) - 1)) : 0;
@@ -310,9 +315,16 @@ int force_go(exfem_block_s* b, const double* u, const double* st_old, double* st
   // 16 bytes, so it takes the arrays themselves to start on one
   const int bulk = ((uintptr_t)st_old % 16 == 0 ? BULK_OLD : 0) | ((uintptr_t)st_new % 16 == 0 ? BULK_NEW : 0) |
                    ((uintptr_t)fe % 16 == 0 ? BULK_FE : 0);
-  force_kernel<ET, J2, MODE, NW><<<(unsigned)((b->ne + per - 1) / per), 32 * NW, smem, s>>>(
-      b->ne, b->X.p, b->conn.p, u, b->scale.p, st_old, st_new, fe, b->tan64.p, b->tan32.p, S, mises, peeq, b->mat,
-      b->lam_e.p, b->mu_e.p, b->order_dev.p, b->tile == 128 ? 7 : 8, bulk, b->dev_err.p, nf, skip);
+  auto kern = force_kernel<ET, J2, MODE, NW>;
+  const unsigned grid = (unsigned)((b->ne + per - 1) / per);
+  if constexpr (MODE == FORCE_PRODUCT)
+    launch_chained(kern, grid, 32 * NW, smem, s, b->ne, b->X.p, b->conn.p, u, b->scale.p, st_old, st_new, fe, b->tan64.p,
+                   b->tan32.p, S, mises, peeq, b->mat, b->lam_e.p, b->mu_e.p, b->order_dev.p, b->tile == 128 ? 7 : 8,
+                   bulk, b->dev_err.p, nf, skip);
+  else
+    kern<<<grid, 32 * NW, smem, s>>>(b->ne, b->X.p, b->conn.p, u, b->scale.p, st_old, st_new, fe, b->tan64.p, b->tan32.p,
+                                     S, mises, peeq, b->mat, b->lam_e.p, b->mu_e.p, b->order_dev.p,
+                                     b->tile == 128 ? 7 : 8, bulk, b->dev_err.p, nf, skip);
   EX_LAUNCH_CHECK();
   return EXFEM_OK;
 }

@@ -40,16 +40,18 @@ struct NodeSmem {
 // Gather of X and u (u may be NULL: zeros) at the nodes of the warp's elements.
 // `eid`: this lane's element; `elem(el)`: the warp's el-th element, called by all lanes;
 // `cnt`: elements of this warp; `nf` (or NULL): per node, the components of u taken as
-// zero (bits).  The caller synchronises the warp afterwards.
+// zero (bits); `ready()`: called by all lanes once, after the loads that depend on the
+// mesh alone and before those of u.  The caller synchronises the warp afterwards.
 //
 // C3D8: a lane loads one of its element's eight nodes and a Walsh-Hadamard transform
 // over the element's lanes turns the corner values into the modal ones (corner signs
 // are the characters of the lane's three bits), so the Gauss points need 7 modes
 // instead of 8 nodes and the centre's gradients are modes themselves.
-template <int ET, bool U, class Elem>
+template <int ET, bool U, class Elem, class Ready>
 __device__ __forceinline__ void gather_nodes(NodeSmem<ET, U>& nd, const double* __restrict__ X,
-                                             const int32_t* __restrict__ conn, const double* __restrict__ u,
-                                             const uint8_t* __restrict__ nf, int64_t eid, int cnt, Elem elem) {
+                                             const int32_t* __restrict__ conn, const double* u,
+                                             const uint8_t* __restrict__ nf, int64_t eid, int cnt, Elem elem,
+                                             Ready ready) {
   constexpr int W = NodeSmem<ET, U>::W, EPW = NodeSmem<ET, U>::EPW, ES = NodeSmem<ET, U>::ES;
   const int lane = threadIdx.x & 31;
   if constexpr (ET == EXFEM_C3D8) {
@@ -59,10 +61,11 @@ __device__ __forceinline__ void gather_nodes(NodeSmem<ET, U>& nd, const double* 
     const unsigned off = U && nf ? nf[node] : 0u;
     double v[W];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      v[c] = X[n3 + c];
-      if constexpr (U) v[3 + c] = u && !((off >> c) & 1u) ? u[n3 + c] : 0.0;
-    }
+    for (int c = 0; c < 3; ++c) v[c] = X[n3 + c];
+    ready();
+    if constexpr (U)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) v[3 + c] = u && !((off >> c) & 1u) ? u[n3 + c] : 0.0;
     // relative to the first node: the sums below then carry no rounding of the
     // distance from the origin
 #pragma unroll
@@ -77,22 +80,32 @@ __device__ __forceinline__ void gather_nodes(NodeSmem<ET, U>& nd, const double* 
 #pragma unroll
     for (int k = 0; k < W; ++k) nd.v[(lane >> 3) * ES + j * W + k] = 0.125 * v[k];
   } else {
-    constexpr int NN = 10;
+    constexpr int NN = 10, P = (EPW * NN + 31) / 32;
+    int32_t node[P];
+    unsigned off[P];
+    int at[P];
 #pragma unroll
-    for (int k0 = 0; k0 < EPW * NN; k0 += 32) {
-      const int k = k0 + lane, el = k / NN < EPW ? k / NN : EPW - 1, a = k - el * NN;
+    for (int p = 0; p < P; ++p) {
+      const int k = 32 * p + lane, el = k / NN < EPW ? k / NN : EPW - 1, a = k - el * NN;
       const int64_t e = elem(el);
-      if (k < cnt * NN) {
-        const int32_t node = conn[e * NN + a];
-        const int64_t n3 = 3 * (int64_t)node;
-        const unsigned off = U && nf ? nf[node] : 0u;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          nd.v[el * ES + a * W + c] = X[n3 + c];
-          if constexpr (U) nd.v[el * ES + a * W + 3 + c] = u && !((off >> c) & 1u) ? u[n3 + c] : 0.0;
-        }
-      }
+      at[p] = k < cnt * NN ? el * ES + a * W : -1;
+      node[p] = at[p] >= 0 ? conn[e * NN + a] : 0;
     }
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      off[p] = U && nf && at[p] >= 0 ? nf[node[p]] : 0u;
+      if (at[p] >= 0)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) nd.v[at[p] + c] = X[3 * (int64_t)node[p] + c];
+    }
+    ready();
+    if constexpr (U)
+#pragma unroll
+      for (int p = 0; p < P; ++p)
+        if (at[p] >= 0)
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+            nd.v[at[p] + 3 + c] = u && !((off[p] >> c) & 1u) ? u[3 * (int64_t)node[p] + c] : 0.0;
   }
 }
 

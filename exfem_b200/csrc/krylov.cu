@@ -89,8 +89,9 @@ __device__ __forceinline__ void block_finish(double v, double* partial, unsigned
 
 template <class T>
 __global__ void __launch_bounds__(RT)
-dot_kernel(int64_t n, const T* __restrict__ a, const T* __restrict__ b, double* partial, unsigned* counter,
+dot_kernel(int64_t n, const T* a, const T* b, double* partial, unsigned* counter,
            PcgScal* sc, double* out, int F, int check_done) {
+  chain_wait();
   if (check_done && sc->done) return;
   // four independent strided loads in flight per thread, four accumulators summed
   // in a fixed order at the end (deterministic for a given grid)
@@ -111,8 +112,9 @@ dot_kernel(int64_t n, const T* __restrict__ a, const T* __restrict__ b, double* 
 
 template <class T>
 __global__ void __launch_bounds__(RT)
-update_xr_kernel(int64_t n, T* __restrict__ x, T* __restrict__ r, const T* __restrict__ p,
-                 const T* __restrict__ Ap, double* partial, unsigned* counter, PcgScal* sc) {
+update_xr_kernel(int64_t n, T* x, T* r, const T* p, const T* Ap, double* partial,
+                 unsigned* counter, PcgScal* sc) {
+  chain_wait();
   if (sc->done) return;
   const T alpha = (T)sc->alpha;
   const int64_t S = (int64_t)gridDim.x * RT;
@@ -145,7 +147,8 @@ update_xr_kernel(int64_t n, T* __restrict__ x, T* __restrict__ r, const T* __res
 }
 
 template <class T>
-__global__ void update_p_kernel(int64_t n, T* __restrict__ p, const T* __restrict__ z, const PcgScal* sc) {
+__global__ void update_p_kernel(int64_t n, T* p, const T* z, const PcgScal* sc) {
+  chain_wait();
   if (sc->done) return;
   const T beta = (T)sc->beta;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -161,16 +164,18 @@ __global__ void convert_kernel(int64_t n, const TS* __restrict__ s, TD* __restri
 }
 
 template <class T>
-__global__ void mask_kernel(int64_t n, const uint8_t* __restrict__ fixed, const T* __restrict__ v,
-                            T* __restrict__ out, const int* __restrict__ skip) {
+__global__ void mask_kernel(int64_t n, const uint8_t* __restrict__ fixed, const T* v, T* out,
+                            const int* skip) {
+  chain_wait();
   if (skip && *skip) return;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     out[i] = fixed[i] ? T(0) : v[i];
 }
 
 template <class T>
-__global__ void pc_out_kernel(int64_t n, const uint8_t* __restrict__ fixed, const T* __restrict__ r,
-                              T* __restrict__ z, const int* __restrict__ skip) {
+__global__ void pc_out_kernel(int64_t n, const uint8_t* __restrict__ fixed, const T* r, T* z,
+                              const int* skip) {
+  chain_wait();
   if (skip && *skip) return;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     if (fixed[i]) z[i] = r[i];
@@ -311,7 +316,8 @@ static unsigned red_grid(int64_t n) {
 
 template <class T>
 static int dot(exfem_solver_s* S, const T* a, const T* b, int F, double* out, int check_done, cudaStream_t st) {
-  dot_kernel<T><<<red_grid(S->n), RT, 0, st>>>(S->n, a, b, S->partial.p, S->counter.p, S->scal.p, out, F, check_done);
+  launch_chained(dot_kernel<T>, red_grid(S->n), RT, 0, st, S->n, a, b, S->partial.p, S->counter.p, S->scal.p, out, F,
+                 check_done);
   EX_LAUNCH_CHECK();
   return EXFEM_OK;
 }
@@ -437,7 +443,7 @@ static int pc_apply(exfem_solver_s* S, const T* r, T* z, const int* skip, cudaSt
   const T* rin = r;
   if (fixed) {
     T* t = ws<T>(S, WT);
-    mask_kernel<T><<<eg, 256, 0, st>>>(n, fixed, r, t, skip);
+    launch_chained(mask_kernel<T>, eg, 256, 0, st, n, fixed, r, t, skip);
     EX_LAUNCH_CHECK();
     rin = t;
   }
@@ -448,7 +454,7 @@ static int pc_apply(exfem_solver_s* S, const T* r, T* z, const int* skip, cudaSt
   int s;
   if ((s = amg_vcycle<T>(S->amg, rin, z, &op0, skip, st))) return s;
   if (fixed) {
-    pc_out_kernel<T><<<eg, 256, 0, st>>>(n, fixed, r, z, skip);
+    launch_chained(pc_out_kernel<T>, eg, 256, 0, st, n, fixed, r, z, skip);
     EX_LAUNCH_CHECK();
   }
   return EXFEM_OK;
@@ -465,11 +471,12 @@ static int pcg_iteration(exfem_solver_s* S, cudaStream_t st, bool looped) {
   int s;
   if ((s = op_apply<T>(S, p, Ap, skip, st))) return s;
   if ((s = dot<T>(S, p, Ap, FIN_ALPHA, nullptr, 1, st))) return s;
-  update_xr_kernel<T><<<red_grid(S->n), RT, 0, st>>>(S->n, x, r, p, Ap, S->partial.p, S->counter.p, S->scal.p);
+  launch_chained(update_xr_kernel<T>, red_grid(S->n), RT, 0, st, S->n, x, r, p, Ap, S->partial.p, S->counter.p,
+                 S->scal.p);
   EX_LAUNCH_CHECK();
   if ((s = pc_apply<T>(S, r, z, skip, st))) return s;
   if ((s = dot<T>(S, r, z, FIN_BETA, nullptr, 1, st))) return s;
-  update_p_kernel<T><<<grid_for(S->n, 256), 256, 0, st>>>(S->n, p, z, S->scal.p);
+  launch_chained(update_p_kernel<T>, grid_for(S->n, 256), 256, 0, st, S->n, p, z, S->scal.p);
   EX_LAUNCH_CHECK();
   return EXFEM_OK;
 }
@@ -839,7 +846,7 @@ int solver_mixed_ru(exfem_solver_s* S, const double* b, double* x, double tol, d
     } else {
       // the iteration that ended the last segment skipped its direction update
       // (p = z + beta p, beta of that iteration): do it with the replaced residual
-      update_p_kernel<float><<<grid_for(n, 256), 256, 0, st>>>(n, p32, z32, S->scal.p);
+      launch_chained(update_p_kernel<float>, grid_for(n, 256), 256, 0, st, n, p32, z32, S->scal.p);
       EX_LAUNCH_CHECK();
     }
     if ((s = dot<float>(S, r32, z32, FIN_RZ0, nullptr, 0, st))) return s;
@@ -977,9 +984,10 @@ static int graph_leaves(cudaGraph_t g, std::vector<cudaGraphNode_t>& out) {
   EX_CUDA(cudaGraphGetNodes(g, nullptr, &nn));
   std::vector<cudaGraphNode_t> nodes(nn);
   if (nn) EX_CUDA(cudaGraphGetNodes(g, nodes.data(), &nn));
-  EX_CUDA(cudaGraphGetEdges(g, nullptr, nullptr, &ne));
+  EX_CUDA(cudaGraphGetEdges_v2(g, nullptr, nullptr, nullptr, &ne));
   std::vector<cudaGraphNode_t> from(ne), to(ne);
-  if (ne) EX_CUDA(cudaGraphGetEdges(g, from.data(), to.data(), &ne));
+  std::vector<cudaGraphEdgeData> kind(ne);  // chained launches leave edges of their own kind
+  if (ne) EX_CUDA(cudaGraphGetEdges_v2(g, from.data(), to.data(), kind.data(), &ne));
   out.clear();
   for (auto nd : nodes)
     if (std::find(from.begin(), from.end(), nd) == from.end()) out.push_back(nd);

@@ -393,15 +393,20 @@ struct TileLayout {
 template <class T, int ET, bool J2, bool ELAME, int TT, int LANES, bool TMA>
 __global__ void __launch_bounds__(TT / LANES, TileLayout<T, ET, TT, LANES, ELAME>::MINB)
 mf_tile_kernel(int64_t ne, int64_t ntile, const T* __restrict__ geo, const uint16_t* __restrict__ lidx,
-               const T* __restrict__ tan, const int32_t* __restrict__ tptr, const int32_t* __restrict__ tpack,
-               const int32_t* __restrict__ tdest, const T* __restrict__ v, T* __restrict__ y, T* __restrict__ part,
-               T lam_m, T mu_m, T K_m, int mu, int vmax, const int* __restrict__ skip, int* __restrict__ err) {
+               const T* tan, const int32_t* __restrict__ tptr, const int32_t* __restrict__ tpack,
+               const int32_t* __restrict__ tdest, const T* v, T* y, T* part,
+               T lam_m, T mu_m, T K_m, int mu, int vmax, const int* skip, int* __restrict__ err) {
   using L = TileLayout<T, ET, TT, LANES, ELAME>;
   using I = typename L::I;
   using P = std::conditional_t<LANES == 2, typename PairOf<T>::type, T>;
   constexpr int NN = L::NN, NG = L::NG, GS = L::GS, NSLOT = L::NSLOT, NT = L::NT, NW = NT / 32;
   constexpr int B = FixedOf<T>::B, GK = 8;
-  if (skip && *skip) return;
+  // the first tile's streams and node list are requested ahead of the wait, except
+  // where the launch may turn out to be skipped (no copy may be in flight at its exit)
+  if (skip) {
+    chain_wait();
+    if (*skip) return;
+  }
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar[2];
   __shared__ T wmax[NW];
@@ -470,6 +475,7 @@ mf_tile_kernel(int64_t ne, int64_t ntile, const T* __restrict__ geo, const uint1
   cur.nu = nxt.nu = 0;
   if ((int64_t)blockIdx.x < ntile) {
     load_ids(tptr[blockIdx.x], tptr[blockIdx.x + 1], cur);
+    if (!skip) chain_wait();
     copies(cur, 0);
   }
   cp_async_commit();
@@ -668,12 +674,11 @@ mf_tile_kernel(int64_t ne, int64_t ntile, const T* __restrict__ geo, const uint1
 // in flight together.
 template <class T>
 __global__ void mf_gather_kernel(int64_t nm, const int32_t* __restrict__ mnodes, const int32_t* __restrict__ mptr,
-                                 const T* __restrict__ part, const T* __restrict__ v, T* __restrict__ y,
-                                 const int* __restrict__ skip) {
+                                 const T* part, const T* v, T* y, const int* skip) {
   // U nodes per thread, the first R entries of each run loaded before any is added
   // (every load in flight at once); entries are still added in run order
   constexpr int U = 4, R = 2;
-  if (skip && *skip) return;
+  bool waited = false;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const Node4<T>* P = reinterpret_cast<const Node4<T>*>(part);
   for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i0 < nm; i0 += U * stride) {
@@ -685,6 +690,11 @@ __global__ void mf_gather_kernel(int64_t nm, const int32_t* __restrict__ mnodes,
       id[u] = i < nm ? (uint32_t)mnodes[i] : 0u;
       q0[u] = i < nm ? mptr[i] : 0;
       q1[u] = i < nm ? mptr[i + 1] : 0;
+    }
+    if (!waited) {  // the lists are constant, the partials are not
+      chain_wait();
+      waited = true;
+      if (skip && *skip) return;
     }
     Node4<T> w[U][R];
 #pragma unroll
@@ -768,9 +778,8 @@ static int mf_go(exfem_block_s* b, const T* geo, const T* tan, const int32_t* tp
   }
   const int64_t grid = std::min<int64_t>(b->ntile, (int64_t)nsm * per_sm);
   const int32_t* tdest = tpack == b->tile_nodes_bc.p ? b->tile_dest_bc.p : b->tile_dest.p;
-  kern<<<(unsigned)grid, L::NT, smem, s>>>(b->ne, b->ntile, geo, b->lidx.p, tan, b->tile_ptr.p, tpack, tdest, v,
-                                           y, part, (T)b->mat.lam, (T)b->mat.mu, (T)b->mat.K, mu, b->vmax, skip,
-                                           b->dev_err.p);
+  launch_chained(kern, (unsigned)grid, L::NT, smem, s, b->ne, b->ntile, geo, b->lidx.p, tan, b->tile_ptr.p, tpack, tdest,
+                 v, y, part, (T)b->mat.lam, (T)b->mat.mu, (T)b->mat.K, mu, b->vmax, skip, b->dev_err.p);
   EX_LAUNCH_CHECK();
   return EXFEM_OK;
 }
@@ -837,8 +846,8 @@ int launch_mf_matvec(exfem_block_s* b, const T* v, T* y, const int* skip, cudaSt
   }
   if (b->nmulti) {
     const int32_t* mn = (bc && b->fixed.p) ? b->multi_nodes_bc.p : b->multi_nodes.p;
-    mf_gather_kernel<T><<<grid_for((b->nmulti + 3) / 4, 256), 256, 0, s>>>(b->nmulti, mn, b->multi_ptr.p, part, v, y,
-                                                                           skip);
+    launch_chained(mf_gather_kernel<T>, grid_for((b->nmulti + 3) / 4, 256), 256, 0, s, b->nmulti, mn, b->multi_ptr.p,
+                   (const T*)part, v, y, skip);
   }
   EX_LAUNCH_CHECK();
   return EXFEM_OK;

@@ -105,7 +105,8 @@ stiffness_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __rest
     for (int k = lane; k < cnt * NG * 19; k += 32) cp_async<8>(sm.st + k, st_old + e0 * (NG * 19) + k, 8);
   }
   const int le = lane / NG, g = lane % NG;
-  gather_nodes<ET, J2>(sm.nd, X, conn, u, nullptr, e0 + (le < cnt ? le : 0), cnt, [&](int el) { return e0 + el; });
+  gather_nodes<ET, J2>(sm.nd, X, conn, u, nullptr, e0 + (le < cnt ? le : 0), cnt, [&](int el) { return e0 + el; },
+                       [] {});
   if constexpr (J2) cp_async_wait_all();
   __syncwarp();
 
