@@ -670,7 +670,8 @@ int amg_set_level_rows(exfem_amg_s* h, size_t l, const double* rho_rows) {
   for (size_t k = 0; k < c.size(); ++k) c32[k] = (float)c[k];
   int st;
   if ((st = L.coef64.upload(c.data(), c.size()))) return st;
-  return L.coef32.upload(c32.data(), c32.size());
+  if ((st = L.coef32.upload(c32.data(), c32.size()))) return st;
+  return uploads_done();
 }
 
 int amg_add_level(exfem_amg_s* h, int64_t n, int64_t nc, const int64_t* Ap, const int32_t* Ai, const double* Av,
@@ -686,7 +687,7 @@ int amg_add_level(exfem_amg_s* h, int64_t n, int64_t nc, const int64_t* Ap, cons
   if ((st = upload_csr(L->R, nc, n, Rp, Ri, Rv))) return st;
   if ((st = L->dinv64.upload(dinv, n))) return st;
   std::vector<float> d32(dinv, dinv + n);
-  if ((st = L->dinv32.upload(d32.data(), n))) return st;
+  if ((st = L->dinv32.upload(d32.data(), n)) || (st = uploads_done())) return st;
   h->levels.push_back(std::move(L));
   return EXFEM_OK;
 }
@@ -791,7 +792,7 @@ int amg_replicate(exfem_amg_s* h, int nmesh, const int64_t* level_offsets, int n
     ua[r] = sa[k];
   }
   if ((st = h->crow_s.upload(us.data(), nu)) || (st = h->crow_m.upload(um.data(), nu)) ||
-      (st = h->crow_a.upload(ua.data(), nu)))
+      (st = h->crow_a.upload(ua.data(), nu)) || (st = uploads_done()))
     return st;
   h->nc = nu;
   h->replicated = true;

@@ -398,7 +398,7 @@ int batch_alloc(exfem_batch_s* B, const int64_t* off_host) {
   for (auto* v : v32)
     if ((s = v->alloc(std::max<int64_t>(B->n, 1)))) return s;
   EX_CUDA(outside_captures([&] { return cudaMallocHost(&B->h_cnt, sizeof(int)); }));
-  return EXFEM_OK;
+  return uploads_done();
 }
 
 }  // namespace exfem

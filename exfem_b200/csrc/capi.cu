@@ -126,7 +126,8 @@ static int init_tangent(exfem_block_s* b) {
     }
   int s;
   if ((s = b->tan64.upload(t.data(), n))) return s;
-  return b->tan32.upload(t32.data(), n);
+  if ((s = b->tan32.upload(t32.data(), n))) return s;
+  return uploads_done();
 }
 
 }  // namespace exfem
@@ -475,7 +476,7 @@ int exfem_block_set_fixed(exfem_block b, const uint8_t* fixed_host) try {
     if (!b->tile_nodes_host.empty())
       EX_CUDA(cudaMemcpy(b->tile_nodes_bc.p, b->tile_nodes_host.data(), b->tile_nodes_host.size() * sizeof(int32_t),
                          cudaMemcpyHostToDevice));
-    return EXFEM_OK;
+    return uploads_done();
   }
   std::vector<uint8_t> f(fixed_host, fixed_host + b->ndof()), nf(b->nn, 0);
   for (int64_t n = 0; n < b->nn; ++n)
@@ -502,10 +503,11 @@ int exfem_block_set_fixed(exfem_block b, const uint8_t* fixed_host) try {
   if (b->fixed.n == (size_t)b->ndof()) {
     EX_CUDA(cudaMemcpy(b->fixed.p, f.data(), f.size(), cudaMemcpyHostToDevice));
     EX_CUDA(cudaMemcpy(b->node_fixed.p, nf.data(), nf.size(), cudaMemcpyHostToDevice));
-    return EXFEM_OK;
+    return uploads_done();
   }
   if ((s = b->fixed.upload(f.data(), f.size()))) return s;
-  return b->node_fixed.upload(nf.data(), nf.size());
+  if ((s = b->node_fixed.upload(nf.data(), nf.size()))) return s;
+  return uploads_done();
 } catch (...) {
   return host_exception();
 }
@@ -634,7 +636,9 @@ int exfem_amg_set_coarse(exfem_amg h, int64_t nc, const double* Ainv) {
   h->crow_s.release();
   h->crow_m.release();
   h->crow_a.release();
-  return h->Ainv.upload(Ainv, (size_t)(nc * nc));
+  int st;
+  if ((st = h->Ainv.upload(Ainv, (size_t)(nc * nc)))) return st;
+  return uploads_done();
 }
 
 int exfem_amg_set_level_rows(exfem_amg h, int level, const double* rho_rows) {
@@ -663,7 +667,8 @@ int exfem_amg_set_coarse_blocks(exfem_amg h, int64_t nblk, const int64_t* offset
   if ((st = h->Ainv.upload(Ainv_blocks, (size_t)a))) return st;
   if ((st = h->crow_s.upload(rs.data(), nc))) return st;
   if ((st = h->crow_m.upload(rm.data(), nc))) return st;
-  return h->crow_a.upload(ra.data(), nc);
+  if ((st = h->crow_a.upload(ra.data(), nc))) return st;
+  return uploads_done();
 } catch (...) {
   return host_exception();
 }

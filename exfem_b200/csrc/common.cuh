@@ -113,6 +113,15 @@ struct DevBuf {
   size_t bytes() const { return n * sizeof(T); }
 };
 
+// DevBuf::upload and cudaMemcpy from pageable memory return once the data is staged:
+// wait for its arrival, so that streams which do not order themselves after the legacy
+// stream may use it.  (That stream only: a device-wide synchronisation would invalidate a
+// graph capture in progress on another host thread.)
+inline int uploads_done() {
+  EX_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+  return EXFEM_OK;
+}
+
 inline unsigned grid_for(size_t n, int block, unsigned cap = 148u * 16u) {
   size_t g = (n + block - 1) / block;
   if (g < 1) g = 1;

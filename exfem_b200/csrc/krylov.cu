@@ -1681,7 +1681,7 @@ int solver_alloc(exfem_solver_s* S) {
   EX_CUDA(cudaMemset(S->counter.p, 0, sizeof(unsigned)));
   if ((s = S->scal.alloc(1))) return s;
   EX_CUDA(outside_captures([&] { return cudaMallocHost(&S->h_scal, sizeof(PcgScal)); }));
-  return EXFEM_OK;
+  return uploads_done();
 }
 
 }  // namespace exfem

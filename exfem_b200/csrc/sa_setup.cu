@@ -390,9 +390,15 @@ __global__ void sa_randn_kernel(int64_t n, uint64_t seed, double* __restrict__ x
 }  // namespace
 namespace {
 
+// upload in stream order: a plain cudaMemcpy from pageable memory returns once the
+// data is staged, and only the legacy stream waits for the rest of its way, so kernels of
+// the set-up's own stream could read the array before it has arrived
 template <class T>
-int up(DevBuf<T>& d, const std::vector<T>& h) {
-  return d.upload(h.empty() ? nullptr : h.data(), h.size());
+int up(DevBuf<T>& d, const std::vector<T>& h, cudaStream_t s) {
+  int st;
+  if ((st = d.alloc(h.size()))) return st;
+  if (!h.empty()) EX_CUDA(cudaMemcpyAsync(d.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, s));
+  return EXFEM_OK;
 }
 
 template <class T>
@@ -429,11 +435,11 @@ struct BlockOp {
   DevBuf<int64_t> ptr;
   DevBuf<int32_t> idx;
   DevBuf<double> val;
-  int set_pattern(Rows&& r) {
+  int set_pattern(Rows&& r, cudaStream_t s) {
     pat = std::move(r);
     int st;
-    if ((st = up(ptr, pat.ptr))) return st;
-    return up(idx, pat.idx);
+    if ((st = up(ptr, pat.ptr, s))) return st;
+    return up(idx, pat.idx, s);
   }
 };
 
@@ -501,8 +507,8 @@ int coarsen(const BlockOp& A, const DevBuf<int32_t>& dagg, const DevBuf<double>&
   DevBuf<int32_t> pidx, qidx, tidx, tslot;
   DevBuf<double> P, AP;
   int st;
-  if ((st = up(pptr, Pp.ptr)) || (st = up(pidx, Pp.idx)) || (st = up(qptr, APp.ptr)) || (st = up(qidx, APp.idx)) ||
-      (st = up(tptr, PT.ptr)) || (st = up(tidx, PT.idx)) || (st = up(tslot, slot)))
+  if ((st = up(pptr, Pp.ptr, s)) || (st = up(pidx, Pp.idx, s)) || (st = up(qptr, APp.ptr, s)) || (st = up(qidx, APp.idx, s)) ||
+      (st = up(tptr, PT.ptr, s)) || (st = up(tidx, PT.idx, s)) || (st = up(tslot, slot, s)))
     return st;
   if ((st = P.alloc(std::max<size_t>(Pp.idx.size() * E, 1))) || (st = AP.alloc(std::max<size_t>(APp.idx.size() * E, 1))) ||
       (st = Ac.val.alloc(std::max<size_t>(Ac.pat.idx.size() * K * K, 1))))
@@ -606,7 +612,7 @@ int blocks_csr_assemble(const std::vector<exfem_block_s*>& blks, const std::vect
     Rows adj;
     if ((st = blocks_adjacency(blks, s, adj))) return st;
     c.nnzb = (int64_t)adj.idx.size();
-    if ((st = up(c.bptr, adj.ptr)) || (st = up(c.bidx, adj.idx)) ||
+    if ((st = up(c.bptr, adj.ptr, s)) || (st = up(c.bidx, adj.idx, s)) ||
         (st = c.bval.alloc(std::max<int64_t>(c.nnzb * 9, 1))))
       return st;
     c.A.n = c.A.ncols = n;
@@ -635,7 +641,7 @@ int block_csr_assemble(exfem_block_s* b, const double* Ke, BlockCsr& c, cudaStre
     Rows adj;
     if ((st = host_node_adjacency(nn, b->ne, b->nnode, conn.data(), adj))) return st;
     c.nnzb = (int64_t)adj.idx.size();
-    if ((st = up(c.bptr, adj.ptr)) || (st = up(c.bidx, adj.idx)) ||
+    if ((st = up(c.bptr, adj.ptr, s)) || (st = up(c.bidx, adj.idx, s)) ||
         (st = c.bval.alloc(std::max<int64_t>(c.nnzb * 9, 1))))
       return st;
     c.A.n = c.A.ncols = n;
@@ -692,7 +698,7 @@ int amg_setup_blocks(exfem_amg_s* h, const std::vector<exfem_block_s*>& blks, co
       return st;
     }
     clk.mark("node adjacency (host)", s, 0);
-    if ((st = A.set_pattern(std::move(adj)))) return st;
+    if ((st = A.set_pattern(std::move(adj), s))) return st;
   }
   if ((st = A.val.alloc(std::max<size_t>(A.pat.idx.size() * 9, 1)))) return st;
   assemble_blocks(blks, Kes, A.nb, A.ptr.p, A.idx.p, A.val.p, s);
@@ -730,13 +736,13 @@ int amg_setup_blocks(exfem_amg_s* h, const std::vector<exfem_block_s*>& blks, co
       if ((int64_t)keep.size() < nblk) {
         DevBuf<int64_t> dkeep;
         DevBuf<double> v;
-        if ((st = up(dkeep, keep)) || (st = v.alloc(std::max<size_t>(keep.size() * bs * bs, 1)))) return st;
+        if ((st = up(dkeep, keep, s)) || (st = v.alloc(std::max<size_t>(keep.size() * bs * bs, 1)))) return st;
         const int64_t nk = (int64_t)keep.size();
         sa_gather_blocks_kernel<<<sa_grid(nk * bs * bs, 256), 256, 0, s>>>(nk, bs * bs, dkeep.p, A.val.p, v.p);
         EX_LAUNCH_CHECK();
         EX_CUDA(cudaStreamSynchronize(s));
         A.val = std::move(v);
-        if ((st = A.set_pattern(std::move(S)))) return st;
+        if ((st = A.set_pattern(std::move(S), s))) return st;
       }
     }
     const int lev = (int)h->levels.size();
@@ -763,10 +769,10 @@ int amg_setup_blocks(exfem_amg_s* h, const std::vector<exfem_block_s*>& blks, co
     BlockOp Ac;
     Ac.bs = K;
     Ac.nb = nagg;
-    if ((st = Ac.set_pattern(std::move(Acp)))) return st;
+    if ((st = Ac.set_pattern(std::move(Acp), s))) return st;
     DevBuf<int32_t> dagg;
     DevBuf<double> dQ;
-    if ((st = up(dagg, agg)) || (st = up(dQ, Q))) return st;
+    if ((st = up(dagg, agg, s)) || (st = up(dQ, Q, s))) return st;
     st = bs == 3 ? coarsen<3>(A, dagg, dQ, dabs, nagg, Pp, APp, PT, slot, Ac, *L, s)
                  : coarsen<6>(A, dagg, dQ, dabs, nagg, Pp, APp, PT, slot, Ac, *L, s);
     if (st) return st;
@@ -819,7 +825,8 @@ int amg_setup_blocks(exfem_amg_s* h, const std::vector<exfem_block_s*>& blks, co
           D[(r * A.bs + i) * nc + (int64_t)A.pat.idx[q] * A.bs + j] = v[(q * A.bs + i) * A.bs + j];
   if ((st = host_coarse_inverse(nc, D, Ainv))) return st;
   clk.mark("coarsest inverse", s, (int)h->levels.size());
-  if ((st = h->Ainv.upload(Ainv.data(), Ainv.size()))) return st;
+  if ((st = up(h->Ainv, Ainv, s))) return st;
+  EX_CUDA(cudaStreamSynchronize(s));  // any stream may use the hierarchy on return
   h->nc = nc;
   h->coarse_nnz = nc * nc;
   return EXFEM_OK;
