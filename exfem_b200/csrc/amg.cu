@@ -335,11 +335,14 @@ template <> const float* csr_vals<float>(const Csr64& A) { return A.v32.p; }
 // ---------------------------------------------------------------- elementwise kernels
 template <class T>
 __global__ void cheb_init0_kernel(int64_t n, const T* b, const T* dinv, T* x, T* r, T* d, T ith,
-                                  const int* skip, const T* __restrict__ rith) {
+                                  const int* skip, const T* __restrict__ rith,
+                                  const uint8_t* __restrict__ fixed, T* masked) {
   chain_wait();
   if (skip && *skip) return;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const T ri = dinv[i] * b[i];
+    const T bi = fixed && fixed[i] ? T(0) : b[i];
+    const T ri = dinv[i] * bi;
+    if (masked) masked[i] = bi;
     x[i] = T(0);
     r[i] = ri;
     d[i] = ri * (rith ? rith[5 * i] : ith);
@@ -349,7 +352,8 @@ __global__ void cheb_init0_kernel(int64_t n, const T* b, const T* dinv, T* x, T*
 template <class T>
 __global__ void cheb_update_kernel(int64_t n, T* x, const T* d, T* r, const T* Ad,
                                    const T* dinv, T* d2, T c1, T c2, const int* skip,
-                                   const T* __restrict__ rc1, const T* __restrict__ rc2, int last) {
+                                   const T* __restrict__ rc1, const T* __restrict__ rc2, int last,
+                                   const uint8_t* __restrict__ fixed, const T* raw) {
   chain_wait();
   if (skip && *skip) return;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -357,7 +361,7 @@ __global__ void cheb_update_kernel(int64_t n, T* x, const T* d, T* r, const T* A
     const T ri = r[i] - dinv[i] * Ad[i];
     const T dn = (rc1 ? rc1[5 * i] : c1) * di + (rc2 ? rc2[5 * i] : c2) * ri;
     if (last) {  // the smoothing's last step: x = (x + d) + d2, r and d2 not kept
-      x[i] = (x[i] + di) + dn;
+      x[i] = fixed && fixed[i] ? raw[i] : (x[i] + di) + dn;
     } else {
       x[i] += di;
       r[i] = ri;
@@ -514,16 +518,36 @@ static int vcycle_level(exfem_amg_s* h, size_t l, const T* b, T* x, const Level0
   const unsigned eg = grid_for(n, 256);
   const T* vals = csr_vals<T>(L.A);
   int st;
+  // level-0 products that run the smoother's steps on their own rows
+  const bool rows = mf && op0->apply_rows && !rc && h->degree > 0;
+  const T* b_raw = b;
+  const uint8_t* fixed = mf && op0->masked ? op0->fixed : nullptr;
   // the last step of the matrix-free and block-sparse smoothings adds the final
   // direction itself (x = (x + d) + d2); the scalar-CSR smoothing adds it after
-  auto smooth_steps = [&]() -> int {
+  auto smooth_steps = [&](bool post) -> int {
     const bool fused_last = mf || useA;
     for (int j = 0; j < h->degree; ++j) {
       const bool last = fused_last && j == h->degree - 1;
-      if (mf) {
+      if (rows) {
+        RowOut<T> o;
+        o.kind = last ? ROW_LAST : ROW_CHEB;
+        o.x = x;
+        o.r = r;
+        o.d2 = d2;
+        o.d = d;
+        o.dinv = dinv;
+        o.c1 = (T)ca[j];
+        o.c2 = (T)cb[j];
+        if (post && last) {
+          o.fixed = fixed;
+          o.raw = b_raw;
+        }
+        if ((st = op0->apply_rows(op0->ctx, d, o, skip, s))) return st;
+      } else if (mf) {
         if ((st = op0->apply(op0->ctx, d, t, skip, s))) return st;
         launch_chained(cheb_update_kernel<T>, eg, 256, 0, s, n, x, d, r, t, dinv, d2, (T)ca[j], (T)cb[j], skip,
-                       rc ? rc + 2 * j : nullptr, rc ? rc + 2 * j + 1 : nullptr, last ? 1 : 0);
+                       rc ? rc + 2 * j : nullptr, rc ? rc + 2 * j + 1 : nullptr, last ? 1 : 0,
+                       post && last ? fixed : nullptr, b_raw);
         EX_LAUNCH_CHECK();
       } else {
         if (useA) {
@@ -547,9 +571,11 @@ static int vcycle_level(exfem_amg_s* h, size_t l, const T* b, T* x, const Level0
     return EXFEM_OK;
   };
   // pre-smoothing from x = 0
-  launch_chained(cheb_init0_kernel<T>, eg, 256, 0, s, n, b, dinv, x, r, d, ith, skip, rc ? rc + 4 : nullptr);
+  launch_chained(cheb_init0_kernel<T>, eg, 256, 0, s, n, b, dinv, x, r, d, ith, skip, rc ? rc + 4 : nullptr,
+                 fixed, fixed ? op0->masked : nullptr);
   EX_LAUNCH_CHECK();
-  if ((st = smooth_steps())) return st;
+  if (fixed) b = op0->masked;
+  if ((st = smooth_steps(false))) return st;
   // residual and restriction
   if (mf) {
     if ((st = op0->apply(op0->ctx, x, t, skip, s))) return st;
@@ -592,7 +618,16 @@ static int vcycle_level(exfem_amg_s* h, size_t l, const T* b, T* x, const Level0
     return st;
   }
   // post-smoothing from the corrected x
-  if (mf) {
+  if (rows) {
+    RowOut<T> o;
+    o.kind = ROW_INIT;
+    o.b = b;
+    o.dinv = dinv;
+    o.r = r;
+    o.d2 = d;
+    o.c1 = ith;
+    if ((st = op0->apply_rows(op0->ctx, x, o, skip, s))) return st;
+  } else if (mf) {
     if ((st = op0->apply(op0->ctx, x, t, skip, s))) return st;
     launch_chained(resinit_kernel<T>, eg, 256, 0, s, n, b, t, dinv, r, d, ith, skip, rc ? rc + 4 : nullptr);
     EX_LAUNCH_CHECK();
@@ -604,7 +639,7 @@ static int vcycle_level(exfem_amg_s* h, size_t l, const T* b, T* x, const Level0
       return st;
     }
   }
-  return smooth_steps();
+  return smooth_steps(true);
 }
 
 template <class T>
@@ -915,7 +950,7 @@ static int vcycle_level_noalloc(exfem_amg_s* h, size_t l, const T* b, T* x, cons
       if (mf) {
         if ((st = op0->apply(op0->ctx, d, t, nullptr, s))) return st;
         cheb_update_kernel<T><<<eg, 256, 0, s>>>(n, x, d, r, t, dinv, d2, (T)ca[j], (T)cb[j], nullptr,
-                                                 rc ? rc + 2 * j : nullptr, rc ? rc + 2 * j + 1 : nullptr, 0);
+                                                 rc ? rc + 2 * j : nullptr, rc ? rc + 2 * j + 1 : nullptr, 0, nullptr, nullptr);
         EX_LAUNCH_CHECK();
       } else {
         if ((st = spmv_lanes<T, SP_CHEB>(L.A, vals, d, r, nullptr, dinv, d2, x, (T)ca[j], (T)cb[j], nullptr, s,
@@ -928,7 +963,7 @@ static int vcycle_level_noalloc(exfem_amg_s* h, size_t l, const T* b, T* x, cons
     EX_LAUNCH_CHECK();
     return EXFEM_OK;
   };
-  cheb_init0_kernel<T><<<eg, 256, 0, s>>>(n, b, dinv, x, r, d, ith, nullptr, rc ? rc + 4 : nullptr);
+  cheb_init0_kernel<T><<<eg, 256, 0, s>>>(n, b, dinv, x, r, d, ith, nullptr, rc ? rc + 4 : nullptr, nullptr, nullptr);
   EX_LAUNCH_CHECK();
   if ((st = smooth_steps())) return st;
   if (mf) {

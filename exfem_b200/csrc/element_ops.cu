@@ -17,8 +17,8 @@ namespace exfem {
 // for 44,541 nodes of C3D8 and 27 us for 176,715 of C3D10.
 __global__ void __launch_bounds__(256)
 gather_assemble_kernel(int64_t ndof, int vmax, const int32_t* __restrict__ plan, int32_t sentinel,
-                       const double* ys, double* f, const uint8_t* __restrict__ fixed, const double* v,
-                       const int* skip) {
+                       const double* ys, const __grid_constant__ RowOut<double> out,
+                       const uint8_t* __restrict__ fixed, const double* v, const int* skip) {
   constexpr int K = 8;
   const int64_t d = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const bool in = d < ndof;
@@ -44,15 +44,18 @@ gather_assemble_kernel(int64_t ndof, int vmax, const int32_t* __restrict__ plan,
       if (slot[k] != sentinel) s += w[k];
     if (slot[K - 1] == sentinel) break;  // slots are listed without gaps
   }
-  f[d] = pass ? v[d] : s;
+  row_out(out, d, pass ? v[d] : s);
 }
 
 int launch_gather_assemble(exfem_block_s* b, const double* ys, double* f, const double* v_opa,
-                           const int* skip, cudaStream_t s) {
+                           const int* skip, cudaStream_t s, const RowOut<double>* out) {
+  RowOut<double> o;
+  if (out) o = *out;
+  else o.y = f;
   if (b->nn == 0) return EXFEM_OK;
   const int threads = 256;
   launch_chained(gather_assemble_kernel, (unsigned)((b->ndof() + threads - 1) / threads), threads, 0, s, b->ndof(),
-                 b->vmax, b->plan.p, (int32_t)(b->ne * b->nnode), ys, f,
+                 b->vmax, b->plan.p, (int32_t)(b->ne * b->nnode), ys, o,
                  (const uint8_t*)(v_opa ? b->fixed.p : nullptr), v_opa, skip);
   EX_LAUNCH_CHECK();
   return EXFEM_OK;
@@ -291,7 +294,7 @@ ebe_rows_kernel(int64_t ne, const int32_t* __restrict__ conn, const double* __re
 }
 
 int launch_ebe_matvec(exfem_block_s* b, const double* Ke, const double* v, double* y,
-                      const int* skip, cudaStream_t s, bool bc) {
+                      const int* skip, cudaStream_t s, bool bc, const RowOut<double>* out) {
   int st;
   if (b->ys.n < (size_t)(b->ne * b->nnode * 3) && (st = b->ys.alloc(b->ne * b->nnode * 3))) return st;
   if (b->ne) {
@@ -309,7 +312,7 @@ int launch_ebe_matvec(exfem_block_s* b, const double* Ke, const double* v, doubl
 #undef EXF_ROWS
     EX_LAUNCH_CHECK();
   }
-  return launch_gather_assemble(b, b->ys.p, y, bc ? v : nullptr, skip, s);
+  return launch_gather_assemble(b, b->ys.p, y, bc ? v : nullptr, skip, s, out);
 }
 
 __global__ void ebe_diag_kernel(int64_t nn, int vmax, int nnode, const int32_t* __restrict__ plan,

@@ -88,18 +88,56 @@ struct Csr64 {  // device CSR, FP64 values and an FP32 copy
   DevBuf<int64_t> rmap, cshift;
 };
 
+// What a product A v does with row i's value: y_i = (A v)_i, or a step of the Chebyshev
+// smoother on the rows it has just formed (no vector A v is stored, no kernel of its own).
+// The gather assembly does this, one thread per row; in the FP32 tiles, whose threads
+// hold three rows each at scattered nodes, it cost more than the kernel it saves (133,623
+// DOF: 176 -> 204 us an iteration).
+//   ROW_CHEB: x += d, r -= dinv (A d), d2 = c1 d + c2 r   (v is the direction d)
+//   ROW_LAST: the same, with the new direction added to x at once (r, d2 not kept);
+//             rows with `fixed` set take `raw`
+//   ROW_INIT: r = dinv (b - A x), d2 = c1 r               (v is x)
+enum RowKind { ROW_SET = 0, ROW_CHEB = 1, ROW_LAST = 2, ROW_INIT = 3 };
+template <class T>
+struct RowOut {
+  int kind = ROW_SET;
+  T *y = nullptr, *x = nullptr, *r = nullptr, *d2 = nullptr;
+  const T *d = nullptr, *b = nullptr, *dinv = nullptr, *raw = nullptr;
+  const uint8_t* fixed = nullptr;
+  T c1 = T(0), c2 = T(0);
+};
+template <class T>
+__device__ __forceinline__ void row_out(const RowOut<T>& o, int64_t i, T v) {
+  if (o.kind == ROW_SET) {
+    o.y[i] = v;
+  } else if (o.kind == ROW_INIT) {
+    const T ri = o.dinv[i] * (o.b[i] - v);
+    o.r[i] = ri;
+    o.d2[i] = ri * o.c1;
+  } else {
+    const T di = o.d[i], ri = o.r[i] - o.dinv[i] * v, dn = o.c1 * di + o.c2 * ri, xi = o.x[i];
+    if (o.kind == ROW_CHEB) {
+      o.x[i] = xi + di;
+      o.r[i] = ri;
+      o.d2[i] = dn;
+    } else {
+      o.x[i] = (o.fixed && o.fixed[i]) ? o.raw[i] : (xi + di) + dn;
+    }
+  }
+}
+
 // element kernels (force.cu, stiffness.cu, element_ops.cu)
 int launch_force(exfem_block_s* b, int mode, const double* u, const double* st_old, double* st_new,
                  double* fe, double* S, double* mises, double* peeq, cudaStream_t s);
 int launch_product_elements(exfem_block_s* b, const double* v, double* fe, bool bc, const int* skip, cudaStream_t s);
 int launch_gather_assemble(exfem_block_s* b, const double* ys, double* f, const double* v_opa,
-                           const int* skip, cudaStream_t s);
+                           const int* skip, cudaStream_t s, const RowOut<double>* out = nullptr);
 int build_geometry(exfem_block_s* b);
 int launch_stiffness(exfem_block_s* b, const double* u, const double* st_old, int dtype, void* Ke,
                      double* ediag, cudaStream_t s, const double* tan_in = nullptr);
 int launch_colour_assemble(exfem_block_s* b, const double* fe, double* f, cudaStream_t s);
 int launch_ebe_matvec(exfem_block_s* b, const double* Ke, const double* v, double* y,
-                      const int* skip, cudaStream_t s, bool bc = true);
+                      const int* skip, cudaStream_t s, bool bc = true, const RowOut<double>* out = nullptr);
 int launch_ebe_diagonal(exfem_block_s* b, const double* Ke, double* diag, cudaStream_t s);
 int launch_geo_stiffness(exfem_block_s* b, const double* S, double* Kg, cudaStream_t s);
 // matrix-free operator (matfree.cu)
@@ -107,6 +145,8 @@ template <class T>
 int launch_mf_matvec(exfem_block_s* b, const T* v, T* y, const int* skip, cudaStream_t s, bool bc = true);
 int launch_mf_diagonal(exfem_block_s* b, double* diag, cudaStream_t s);
 bool product_by_points(int etype, int64_t ne);  // FP64 products through element vectors
+int launch_product_points(exfem_block_s* b, const double* v, double* y, const int* skip, cudaStream_t s, bool bc,
+                          const RowOut<double>* out);
 // bounded device waits: read and clear a block's wait-failure flag (capi.cu); a
 // kernel whose only wait can never complete (matfree.cu)
 int block_wait_status(exfem_block_s* b, cudaStream_t s);

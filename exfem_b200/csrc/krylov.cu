@@ -400,6 +400,24 @@ static int op0_apply(void* ctx, const T* x, T* y, const int* skip, cudaStream_t 
   return op_apply<T>((exfem_solver_s*)ctx, x, y, skip, st);
 }
 
+// smoother steps on the product's own rows: FP64 products of one block whose rows come
+// out of the gather assembly
+static bool has_rows(const exfem_solver_s* S) {
+  if (!S->more.empty()) return false;
+  if (S->op == EXFEM_OP_EBE_F64) return true;
+  const exfem_block_s* b = S->blk;
+  return S->op != EXFEM_OP_CSR_F64 && product_by_points(b->etype, b->ne) && (b->etype == EXFEM_C3D8 || b->affine);
+}
+
+static int op0_rows(void* ctx, const double* x, const RowOut<double>& out, const int* skip, cudaStream_t st) {
+  auto* S = (exfem_solver_s*)ctx;
+  if (S->op == EXFEM_OP_EBE_F64) {
+    if (!S->Ke) { set_error("solver: stored-Ke operator without Ke (call exfem_solver_set_ke)"); return EXFEM_ERR_ARG; }
+    return launch_ebe_matvec(S->blk, S->Ke, x, nullptr, skip, st, true, &out);
+  }
+  return launch_product_points(S->blk, x, nullptr, skip, st, true, &out);
+}
+
 template <class T>
 static int pc_apply(exfem_solver_s* S, const T* r, T* z, const int* skip, cudaStream_t st) {
   const int64_t n = S->n;
@@ -441,7 +459,9 @@ static int pc_apply(exfem_solver_s* S, const T* r, T* z, const int* skip, cudaSt
   }
   const uint8_t* fixed = S->blk->fixed.p;
   const T* rin = r;
-  if (fixed) {
+  // the V-cycle's mesh level masks and restores the prescribed DOFs itself
+  const bool inside = !S->amg->levels.empty() && !S->amg->levels[0]->coef64.p && S->amg->degree > 0;
+  if (fixed && !inside) {
     T* t = ws<T>(S, WT);
     launch_chained(mask_kernel<T>, eg, 256, 0, st, n, fixed, r, t, skip);
     EX_LAUNCH_CHECK();
@@ -451,9 +471,15 @@ static int pc_apply(exfem_solver_s* S, const T* r, T* z, const int* skip, cudaSt
   op0.apply = &op0_apply<T>;
   op0.ctx = S;
   op0.dinv = sdinv<T>(S);
+  if (inside && fixed) {
+    op0.fixed = fixed;
+    op0.masked = ws<T>(S, WT);
+  }
+  if constexpr (sizeof(T) == 8)
+    if (has_rows(S)) op0.apply_rows = &op0_rows;
   int s;
   if ((s = amg_vcycle<T>(S->amg, rin, z, &op0, skip, st))) return s;
-  if (fixed) {
+  if (fixed && !inside) {
     launch_chained(pc_out_kernel<T>, eg, 256, 0, st, n, fixed, r, z, skip);
     EX_LAUNCH_CHECK();
   }

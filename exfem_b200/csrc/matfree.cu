@@ -813,6 +813,13 @@ static int mf_dispatch(exfem_block_s* b, const T* geo, const T* tan, const int32
 // elements 8.6 / 34, 113,724 38 / 70, 384,000 135 / 136, 1,053,696 380 / 343 (J2 alike).
 bool product_by_points(int etype, int64_t ne) { return ne <= (etype == EXFEM_C3D8 ? 120000 : 350000); }
 
+int launch_product_points(exfem_block_s* b, const double* v, double* y, const int* skip, cudaStream_t s, bool bc,
+                          const RowOut<double>* out) {
+  const int st = launch_product_elements(b, v, b->ys_product(), bc, skip, s);
+  if (st) return st;
+  return launch_gather_assemble(b, b->ys_product(), y, bc ? v : nullptr, skip, s, out);
+}
+
 template <class T>
 int launch_mf_matvec(exfem_block_s* b, const T* v, T* y, const int* skip, cudaStream_t s, bool bc) {
   const int64_t ndof = b->ndof();
@@ -823,9 +830,7 @@ int launch_mf_matvec(exfem_block_s* b, const T* v, T* y, const int* skip, cudaSt
   }
   if constexpr (sizeof(T) == 8) {
     if (product_by_points(b->etype, b->ne)) {
-      const int st = launch_product_elements(b, v, b->ys_product(), bc, skip, s);
-      if (st) return st;
-      return launch_gather_assemble(b, b->ys_product(), y, bc ? v : nullptr, skip, s);
+      return launch_product_points(b, v, y, skip, s, bc, nullptr);
     }
   }
   T* part = reinterpret_cast<T*>(b->partial.p);

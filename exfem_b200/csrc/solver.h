@@ -62,6 +62,12 @@ struct Level0Op {
   int (*apply)(void* ctx, const T* x, T* y, const int* skip, cudaStream_t s) = nullptr;
   void* ctx = nullptr;
   const T* dinv = nullptr;
+  // the product whose rows go into a smoother step (RowOut), where the operator has it
+  int (*apply_rows)(void* ctx, const T* x, const RowOut<T>& out, const int* skip, cudaStream_t s) = nullptr;
+  // prescribed DOFs (or NULL), whose right-hand side counts as zero (kept in `masked`)
+  // and whose result is the right-hand side itself; not with per-row coefficients
+  const uint8_t* fixed = nullptr;
+  T* masked = nullptr;
 };
 
 template <class T>
