@@ -570,9 +570,63 @@ int solver_refresh_diagonal(exfem_solver_s* S, cudaStream_t st) {
   return EXFEM_OK;
 }
 
-// Graph of the whole PCG loop: a head kernel sets the loop condition from the
-// device scalars, then a conditional while node runs one captured iteration plus
-// the condition kernel until the recursion is done (or maxiter + 2 passes)
+// nodes of g that no edge leaves
+static int graph_leaves(cudaGraph_t g, std::vector<cudaGraphNode_t>& out) {
+  size_t nn = 0, ne = 0;
+  EX_CUDA(cudaGraphGetNodes(g, nullptr, &nn));
+  std::vector<cudaGraphNode_t> nodes(nn);
+  if (nn) EX_CUDA(cudaGraphGetNodes(g, nodes.data(), &nn));
+  EX_CUDA(cudaGraphGetEdges_v2(g, nullptr, nullptr, nullptr, &ne));
+  std::vector<cudaGraphNode_t> from(ne), to(ne);
+  std::vector<cudaGraphEdgeData> kind(ne);  // chained launches leave edges of their own kind
+  if (ne) EX_CUDA(cudaGraphGetEdges_v2(g, from.data(), to.data(), kind.data(), &ne));
+  out.clear();
+  for (auto nd : nodes)
+    if (std::find(from.begin(), from.end(), nd) == from.end()) out.push_back(nd);
+  return EXFEM_OK;
+}
+
+// capture the work of f on stream st into g after the nodes deps
+template <class F>
+static int capture_into(cudaGraph_t g, const std::vector<cudaGraphNode_t>& deps, cudaStream_t st, F f) {
+  cudaError_t e = cudaStreamBeginCaptureToGraph(st, g, deps.empty() ? nullptr : deps.data(), nullptr, deps.size(),
+                                                cudaStreamCaptureModeThreadLocal);
+  if (e != cudaSuccess) {
+    set_error("graph capture could not start: %s", cudaGetErrorString(e));
+    return EXFEM_ERR_CUDA;
+  }
+  int cs = f();
+  if (!cs && cudaGetLastError() != cudaSuccess) cs = EXFEM_ERR_CUDA;
+  cudaGraph_t out = nullptr;
+  e = cudaStreamEndCapture(st, &out);
+  if (cs) return cs;
+  if (e != cudaSuccess) {
+    set_error("graph capture failed: %s", cudaGetErrorString(e));
+    return EXFEM_ERR_CUDA;
+  }
+  return EXFEM_OK;
+}
+
+// start of a PCG recursion on the workspace vectors (tolerance and budget already in the
+// scalars): x = 0, r = b, z = M(r), p = z and the first scalars
+template <class T>
+static int pcg_start(exfem_solver_s* S, cudaStream_t st) {
+  const int64_t n = S->n;
+  T *x = ws<T>(S, WX), *r = ws<T>(S, WR), *z = ws<T>(S, WZ), *p = ws<T>(S, WP), *b = ws<T>(S, WB);
+  int s;
+  EX_CUDA(cudaMemsetAsync(x, 0, sizeof(T) * n, st));
+  EX_CUDA(cudaMemcpyAsync(r, b, sizeof(T) * n, cudaMemcpyDeviceToDevice, st));
+  if ((s = dot<T>(S, b, b, FIN_BB, nullptr, 0, st))) return s;
+  if ((s = pc_apply<T>(S, r, z, nullptr, st))) return s;
+  EX_CUDA(cudaMemcpyAsync(p, z, sizeof(T) * n, cudaMemcpyDeviceToDevice, st));
+  if ((s = dot<T>(S, r, z, FIN_RZ0, nullptr, 0, st))) return s;
+  return dot<T>(S, r, r, FIN_RR0, nullptr, 0, st);
+}
+
+// Graph of a whole PCG solve: the start, a head kernel that sets the loop condition from
+// the device scalars, and a conditional while node that runs one captured iteration plus
+// the condition kernel until the recursion is done (or maxiter + 2 passes).  (With the
+// start's 40 launches outside, they were a fifth of a 1,575-DOF solve.)
 template <class T>
 static int loop_graph(exfem_solver_s* S, cudaStream_t st, cudaGraph_t* out) {
   cudaGraph_t g = nullptr;
@@ -586,37 +640,35 @@ static int loop_graph(exfem_solver_s* S, cudaStream_t st, cudaGraph_t* out) {
   cudaError_t e = cudaGraphConditionalHandleCreate(&h, g, 0, 0);
   if (e != cudaSuccess) return fail(e, "condition handle");
   PcgScal* sc = S->scal.p;
-  int head = 1;
-  void* args[] = {&h, &sc, &head};
-  cudaKernelNodeParams kp = {};
-  kp.func = (void*)loop_cond_kernel;
-  kp.gridDim = dim3(1);
-  kp.blockDim = dim3(1);
-  kp.kernelParams = args;
-  cudaGraphNode_t n_head, n_loop;
-  if ((e = cudaGraphAddKernelNode(&n_head, g, nullptr, 0, &kp)) != cudaSuccess) return fail(e, "head node");
+  int cs = capture_into(g, {}, st, [&]() -> int {
+    int q;
+    if ((q = pcg_start<T>(S, st))) return q;
+    loop_cond_kernel<<<1, 1, 0, st>>>(h, sc, 1);
+    return EXFEM_OK;
+  });
+  std::vector<cudaGraphNode_t> leaves;
+  if (!cs) cs = graph_leaves(g, leaves);
+  if (cs) {
+    cudaGraphDestroy(g);
+    return cs;
+  }
+  cudaGraphNode_t n_loop;
   cudaGraphNodeParams cp = {};
   cp.type = cudaGraphNodeTypeConditional;
   cp.conditional.handle = h;
   cp.conditional.type = cudaGraphCondTypeWhile;
   cp.conditional.size = 1;
-  if ((e = cudaGraphAddNode(&n_loop, g, &n_head, 1, &cp)) != cudaSuccess) return fail(e, "while node");
-  cudaGraph_t body = cp.conditional.phGraph_out[0];
-  if ((e = cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
-      cudaSuccess)
-    return fail(e, "capture of the loop body");
-  int cs = pcg_iteration<T>(S, st, true);
-  if (!cs) {
+  if ((e = cudaGraphAddNode(&n_loop, g, leaves.data(), leaves.size(), &cp)) != cudaSuccess) return fail(e, "while node");
+  cs = capture_into(cp.conditional.phGraph_out[0], {}, st, [&]() -> int {
+    int q;
+    if ((q = pcg_iteration<T>(S, st, true))) return q;
     loop_cond_kernel<<<1, 1, 0, st>>>(h, sc, 0);
-    if (cudaGetLastError() != cudaSuccess) cs = EXFEM_ERR_CUDA;
-  }
-  cudaGraph_t captured = nullptr;
-  e = cudaStreamEndCapture(st, &captured);
+    return EXFEM_OK;
+  });
   if (cs) {
     cudaGraphDestroy(g);
     return cs;
   }
-  if (e != cudaSuccess) return fail(e, "end of the body capture");
   *out = g;
   return EXFEM_OK;
 }
@@ -689,18 +741,15 @@ static int pcg_chunks(exfem_solver_s* S, int maxiter, cudaStream_t st) {
   const int gi = sizeof(T) == 8 ? 0 : 1;
   const int chunk = S->chunk > 0 ? S->chunk : 8;
   int s;
-  if (S->use_graph && S->gexec[gi] && S->gloop[gi]) {  // one launch runs the loop to the end
-    EX_CUDA(cudaGraphLaunch(S->gexec[gi], st));
-    EX_CUDA(cudaMemcpyAsync(S->h_scal, S->scal.p, sizeof(PcgScal), cudaMemcpyDeviceToHost, st));
-    EX_CUDA(cudaStreamSynchronize(st));
-    return EXFEM_OK;
-  }
+  // (a graph of the whole solve starts its own recursion: segments that continue one are
+  // launched kernel by kernel)
+  const bool graph = S->use_graph && !S->gloop[gi];
   const int max_chunks = maxiter / chunk + 2;
   for (int c = 0; c < max_chunks; ++c) {
     EX_CUDA(cudaMemcpyAsync(S->h_scal, S->scal.p, sizeof(PcgScal), cudaMemcpyDeviceToHost, st));
     EX_CUDA(cudaStreamSynchronize(st));
     if (S->h_scal->done) break;
-    if (S->use_graph) {
+    if (graph) {
       EX_CUDA(cudaGraphLaunch(S->gexec[gi], st));
     } else {
       for (int i = 0; i < chunk; ++i)
@@ -718,17 +767,17 @@ static int pcg_run(exfem_solver_s* S, double tol, int maxiter, int* iters, doubl
   const int64_t n = S->n;
   int s;
   if ((s = pcg_prepare<T>(S, st))) return s;
-  T *x = ws<T>(S, WX), *r = ws<T>(S, WR), *z = ws<T>(S, WZ), *p = ws<T>(S, WP), *b = ws<T>(S, WB);
   init_scal_kernel<<<1, 1, 0, st>>>(S->scal.p, tol, maxiter);
   EX_LAUNCH_CHECK();
-  EX_CUDA(cudaMemsetAsync(x, 0, sizeof(T) * n, st));
-  EX_CUDA(cudaMemcpyAsync(r, b, sizeof(T) * n, cudaMemcpyDeviceToDevice, st));
-  if ((s = dot<T>(S, b, b, FIN_BB, nullptr, 0, st))) return s;
-  if ((s = pc_apply<T>(S, r, z, nullptr, st))) return s;
-  EX_CUDA(cudaMemcpyAsync(p, z, sizeof(T) * n, cudaMemcpyDeviceToDevice, st));
-  if ((s = dot<T>(S, r, z, FIN_RZ0, nullptr, 0, st))) return s;
-  if ((s = dot<T>(S, r, r, FIN_RR0, nullptr, 0, st))) return s;
-  if ((s = pcg_chunks<T>(S, maxiter, st))) return s;
+  const int gi = sizeof(T) == 8 ? 0 : 1;
+  if (S->use_graph && S->gexec[gi] && S->gloop[gi]) {  // one launch runs the solve to the end
+    EX_CUDA(cudaGraphLaunch(S->gexec[gi], st));
+    EX_CUDA(cudaMemcpyAsync(S->h_scal, S->scal.p, sizeof(PcgScal), cudaMemcpyDeviceToHost, st));
+    EX_CUDA(cudaStreamSynchronize(st));
+  } else {
+    if ((s = pcg_start<T>(S, st))) return s;
+    if ((s = pcg_chunks<T>(S, maxiter, st))) return s;
+  }
   const PcgScal& h = *S->h_scal;
   if (iters) *iters = h.k;
   const double rel = sqrt(h.rr / fmax(h.bb, 1e-300));
@@ -1002,43 +1051,6 @@ __global__ void mx_cond_kernel(cudaGraphConditionalHandle h, MixedScal* ms, int 
   else ms->loops += 1;
   const bool more = !ms->done && (long long)ms->loops <= (long long)ms->max_updates;
   cudaGraphSetConditional(h, more ? 1u : 0u);
-}
-
-// nodes of g that no edge leaves
-static int graph_leaves(cudaGraph_t g, std::vector<cudaGraphNode_t>& out) {
-  size_t nn = 0, ne = 0;
-  EX_CUDA(cudaGraphGetNodes(g, nullptr, &nn));
-  std::vector<cudaGraphNode_t> nodes(nn);
-  if (nn) EX_CUDA(cudaGraphGetNodes(g, nodes.data(), &nn));
-  EX_CUDA(cudaGraphGetEdges_v2(g, nullptr, nullptr, nullptr, &ne));
-  std::vector<cudaGraphNode_t> from(ne), to(ne);
-  std::vector<cudaGraphEdgeData> kind(ne);  // chained launches leave edges of their own kind
-  if (ne) EX_CUDA(cudaGraphGetEdges_v2(g, from.data(), to.data(), kind.data(), &ne));
-  out.clear();
-  for (auto nd : nodes)
-    if (std::find(from.begin(), from.end(), nd) == from.end()) out.push_back(nd);
-  return EXFEM_OK;
-}
-
-// capture the work of f on stream st into g after the nodes deps
-template <class F>
-static int capture_into(cudaGraph_t g, const std::vector<cudaGraphNode_t>& deps, cudaStream_t st, F f) {
-  cudaError_t e = cudaStreamBeginCaptureToGraph(st, g, deps.empty() ? nullptr : deps.data(), nullptr, deps.size(),
-                                                cudaStreamCaptureModeThreadLocal);
-  if (e != cudaSuccess) {
-    set_error("graph capture could not start: %s", cudaGetErrorString(e));
-    return EXFEM_ERR_CUDA;
-  }
-  int cs = f();
-  if (!cs && cudaGetLastError() != cudaSuccess) cs = EXFEM_ERR_CUDA;
-  cudaGraph_t out = nullptr;
-  e = cudaStreamEndCapture(st, &out);
-  if (cs) return cs;
-  if (e != cudaSuccess) {
-    set_error("graph capture failed: %s", cudaGetErrorString(e));
-    return EXFEM_ERR_CUDA;
-  }
-  return EXFEM_OK;
 }
 
 // the nodes of one reliable-update solve of mx_b into mx_x, appended to g after its
