@@ -15,7 +15,7 @@
 // J2 blocks are walked in tile order, in which the tangent data of neighbouring
 // elements are neighbours in memory; otherwise elements are taken as they are numbered.
 //
-// Measured on B200, with the assembly: 40,000 J2 C3D8 51 us, 125,550 J2 C3D10 89 us
+// Measured on B200, with the assembly: 40,000 J2 C3D8 49 us, 125,550 J2 C3D10 88 us
 // (states read and written, tangent data written); one thread per element, which read
 // each state entry with a stride of a whole element, took 170 and 212 us, and copying
 // states entry by entry instead of in bulk 63 and 104 us.
