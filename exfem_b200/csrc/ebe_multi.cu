@@ -297,7 +297,6 @@ int multi_go(exfem_block_s* b, const KT* Ke, const VT* V, VT* ys, const uint8_t*
   auto kern = ebe_multi_kernel<ET, NR, KT, VT, NW>;
   if constexpr (smem > 48 * 1024)
     EX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  EX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
   kern<<<(unsigned)((b->ne + per - 1) / per), 32 * NW, smem, s>>>(b->ne, b->conn.p, Ke, V, fx, ys,
                                                                    (uintptr_t)V % 16 == 0, (uintptr_t)Ke % 16 == 0,
                                                                    b->dev_err.p);

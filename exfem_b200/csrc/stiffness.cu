@@ -337,7 +337,11 @@ int stiffness_go(exfem_block_s* b, const double* u, const double* st_old, const 
   auto kern = stiffness_kernel<ET, J2, MODE, OutT, NW>;
   if constexpr (smem > 48 * 1024)
     EX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  EX_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  // No preferred split of the on-chip memory is set: a launch that wants another split than
+  // the running kernels' waits for them to leave, and under other streams' solves (device
+  // loops) that is the end of their backlog.  J2 Newton corrections take their diagonal
+  // from here: mean J2 service at 2,000 requests/s on 24 streams 20 s with the preference,
+  // 2.4 s without.  Alone the kernel is no slower (40,000 J2 C3D8: 65.5 and 63.5 us).
   constexpr size_t bytes = (size_t)S::ND * S::ND * sizeof(OutT);
   const int bulk = MODE == 0 && bytes % 16 == 0 && (uintptr_t)Ke % 16 == 0;
   const int64_t per = NW * S::EPW;
