@@ -23,7 +23,7 @@ namespace exfem {
 constexpr int RT = 256;          // reduction block size
 constexpr int RED_MAX_BLOCKS = 592;   // 4 CTAs of 256 per SM
 
-enum Fin { FIN_BB = 0, FIN_RZ0, FIN_RR0, FIN_ALPHA, FIN_RR, FIN_BETA, FIN_STORE };
+enum Fin { FIN_BB = 0, FIN_RZ0, FIN_RR0, FIN_ALPHA, FIN_RR, FIN_BETA, FIN_BETA_CONJ, FIN_STORE };
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -31,7 +31,8 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-__device__ __forceinline__ void fin_apply(int F, double s, PcgScal* sc, double* out) {
+// s2: the second sum of FIN_BETA_CONJ
+__device__ __forceinline__ void fin_apply(int F, double s, double s2, PcgScal* sc, double* out) {
   switch (F) {
     case FIN_BB:
       sc->bb = s;
@@ -48,7 +49,9 @@ __device__ __forceinline__ void fin_apply(int F, double s, PcgScal* sc, double* 
       break;
     case FIN_RR: sc->rr = s; break;
     case FIN_BETA:
+    case FIN_BETA_CONJ:
       sc->beta = s / sc->rz;
+      if (F == FIN_BETA_CONJ && !(sc->beta >= 0.0 && sc->beta <= 1.0)) sc->beta = -s2 / sc->pAp;
       sc->rz = s;
       sc->k += 1;
       sc->done = !(sc->rr > sc->tol2 && sc->k < sc->maxiter);
@@ -57,19 +60,26 @@ __device__ __forceinline__ void fin_apply(int F, double s, PcgScal* sc, double* 
   }
 }
 
-// block partial sums + last-block final sum in index order
-__device__ __forceinline__ void block_finish(double v, double* partial, unsigned* counter, int F,
+// block partial sums + last-block final sum in index order, of M sums at once
+template <int M>
+__device__ __forceinline__ void block_finish(double (&v)[M], double* partial, unsigned* counter, int F,
                                              PcgScal* sc, double* out) {
-  __shared__ double sw[RT / 32];
+  __shared__ double sw[M][RT / 32];
   __shared__ int last;
-  v = warp_sum(v);
-  if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = v;
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    v[m] = warp_sum(v[m]);
+    if ((threadIdx.x & 31) == 0) sw[m][threadIdx.x >> 5] = v[m];
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
-    double t = 0.0;
 #pragma unroll
-    for (int w = 0; w < RT / 32; ++w) t += sw[w];
-    partial[blockIdx.x] = t;
+    for (int m = 0; m < M; ++m) {
+      double t = 0.0;
+#pragma unroll
+      for (int w = 0; w < RT / 32; ++w) t += sw[m][w];
+      partial[m * gridDim.x + blockIdx.x] = t;
+    }
     __threadfence();
     const unsigned tk = atomicAdd(counter, 1u);
     last = (tk == gridDim.x - 1);
@@ -77,11 +87,15 @@ __device__ __forceinline__ void block_finish(double v, double* partial, unsigned
   __syncthreads();
   if (last && threadIdx.x < 32) {
     __threadfence();
-    double t = 0.0;
-    for (unsigned i = threadIdx.x; i < gridDim.x; i += 32) t += ((volatile double*)partial)[i];
-    t = warp_sum(t);
+    double t[M];
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      t[m] = 0.0;
+      for (unsigned i = threadIdx.x; i < gridDim.x; i += 32) t[m] += ((volatile double*)partial)[m * gridDim.x + i];
+      t[m] = warp_sum(t[m]);
+    }
     if (threadIdx.x == 0) {
-      fin_apply(F, t, sc, out);
+      fin_apply(F, t[0], t[M - 1], sc, out);
       *counter = 0u;
     }
   }
@@ -107,7 +121,39 @@ dot_kernel(int64_t n, const T* a, const T* b, double* partial, unsigned* counter
     a3 += (double)x3 * (double)y3;
   }
   for (; i < n; i += S) a0 += (double)a[i] * (double)b[i];
-  block_finish((a0 + a1) + (a2 + a3), partial, counter, F, sc, out);
+  double v[1] = {(a0 + a1) + (a2 + a3)};
+  block_finish(v, partial, counter, F, sc, out);
+}
+
+// r.z and z.Ap in one pass, for the new direction of the FP32 recursion (FIN_BETA_CONJ)
+template <class T>
+__global__ void __launch_bounds__(RT)
+dot_conj_kernel(int64_t n, const T* z, const T* r, const T* Ap, double* partial, unsigned* counter, PcgScal* sc) {
+  chain_wait();
+  if (sc->done) return;
+  const int64_t S = (int64_t)gridDim.x * RT;
+  double a[4] = {0.0, 0.0, 0.0, 0.0}, c[4] = {0.0, 0.0, 0.0, 0.0};
+  int64_t i = blockIdx.x * (int64_t)RT + threadIdx.x;
+  for (; i + 3 * S < n; i += 4 * S) {
+    T x[4], y[4], w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      x[k] = z[i + k * S];
+      y[k] = r[i + k * S];
+      w[k] = Ap[i + k * S];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      a[k] += (double)x[k] * (double)y[k];
+      c[k] += (double)x[k] * (double)w[k];
+    }
+  }
+  for (; i < n; i += S) {
+    a[0] += (double)z[i] * (double)r[i];
+    c[0] += (double)z[i] * (double)Ap[i];
+  }
+  double v[2] = {(a[0] + a[1]) + (a[2] + a[3]), (c[0] + c[1]) + (c[2] + c[3])};
+  block_finish(v, partial, counter, FIN_BETA_CONJ, sc, nullptr);
 }
 
 template <class T>
@@ -143,7 +189,8 @@ update_xr_kernel(int64_t n, T* x, T* r, const T* p, const T* Ap, double* partial
     r[i] = ri;
     acc[0] += (double)ri * (double)ri;
   }
-  block_finish((acc[0] + acc[1]) + (acc[2] + acc[3]), partial, counter, FIN_RR, sc, nullptr);
+  double v[1] = {(acc[0] + acc[1]) + (acc[2] + acc[3])};
+  block_finish(v, partial, counter, FIN_RR, sc, nullptr);
 }
 
 template <class T>
@@ -490,6 +537,18 @@ static int pc_apply(exfem_solver_s* S, const T* r, T* z, const int* skip, cudaSt
 // flag; the body of a device-side loop runs only while the flag is unset, so its
 // products and V-cycle need not (about half a microsecond of each kernel's latency,
 // some 35 kernels an iteration).
+//
+// beta = r.z / (r.z)_old and -z.Ap / p.Ap are the same number in exact arithmetic.  The
+// FP32 recursion takes the second, which makes the new direction conjugate to the last one
+// as the product has it, where the first lies outside [0, 1]: the V-cycle is indefinite on
+// some vectors of a mesh with strongly varying moduli, r.z passes through zero there, and
+// dividing by it gives directions (beta 62 was met) that hold little but rounding.  Inside
+// [0, 1] r.z falls as it should and the first is the better determined one: after a large
+// drop z.Ap is a small difference of large terms (on a mesh with an exact preconditioner it
+// led to non-finite steps).  C3D10 cubes with moduli over a decade, cg_tol 1e-8, FP32
+// iterations with the first form alone and now: 12.5M DOF, five seeds, 131 201 82 152 104
+// and 93 116 82 138 95; 1.6M DOF, four seeds, 102 69 63 64 and 78 70 61 62; where r.z never
+// rises the iterates are the same.
 template <class T>
 static int pcg_iteration(exfem_solver_s* S, cudaStream_t st, bool looped) {
   const int* skip = looped ? nullptr : &S->scal.p->done;
@@ -501,7 +560,12 @@ static int pcg_iteration(exfem_solver_s* S, cudaStream_t st, bool looped) {
                  S->scal.p);
   EX_LAUNCH_CHECK();
   if ((s = pc_apply<T>(S, r, z, skip, st))) return s;
-  if ((s = dot<T>(S, r, z, FIN_BETA, nullptr, 1, st))) return s;
+  if constexpr (sizeof(T) == 8) {
+    if ((s = dot<T>(S, r, z, FIN_BETA, nullptr, 1, st))) return s;
+  } else {
+    launch_chained(dot_conj_kernel<T>, red_grid(S->n), RT, 0, st, S->n, z, r, Ap, S->partial.p, S->counter.p, S->scal.p);
+    EX_LAUNCH_CHECK();
+  }
   launch_chained(update_p_kernel<T>, grid_for(S->n, 256), 256, 0, st, S->n, p, z, S->scal.p);
   EX_LAUNCH_CHECK();
   return EXFEM_OK;
@@ -1713,7 +1777,7 @@ int solver_alloc(exfem_solver_s* S) {
     for (auto* v : c32)
       if ((s = v->alloc(std::max<int64_t>(n, 1)))) return s;
   }
-  if ((s = S->partial.alloc(RED_MAX_BLOCKS))) return s;
+  if ((s = S->partial.alloc(2 * RED_MAX_BLOCKS))) return s;  // two sums at most (dot_conj_kernel)
   if ((s = S->dscr.alloc(4))) return s;
   if ((s = S->counter.alloc(1))) return s;
   EX_CUDA(cudaMemset(S->counter.p, 0, sizeof(unsigned)));
