@@ -119,6 +119,7 @@ _SIGS = {
     "exfem_amg_export_coarse": ([VP, P, P], C.c_int),
     "exfem_solver_set_mixed_mode": ([VP, I32, D], C.c_int),
     "exfem_selftest_bounded_wait": ([I32, VP], C.c_int),
+    "exfem_selftest_block_wait": ([VP, I32, VP], C.c_int),
     "exfem_block_tile_conn": ([VP, P], C.c_int),
     "exfem_queue_create": ([I32, C.POINTER(VP)], C.c_int),
     "exfem_queue_destroy": ([VP], C.c_int),

@@ -446,7 +446,11 @@ int exfem_batch_solve(exfem_batch b, const double* rhs, double* x, double tol, d
     EX_CUDA(cudaEventRecord(ev, user));
     EX_CUDA(cudaStreamWaitEvent(work, ev, 0));
   }
-  const int s = batch_solve(b, rhs, x, tol, inner_tol, max_pass, maxiter, iters, passes, relres, work);
+  int s = batch_solve(b, rhs, x, tol, inner_tol, max_pass, maxiter, iters, passes, relres, work);
+  if (s >= 0) {
+    const int w = block_wait_status(b->blk, work);
+    if (w < 0) s = w;
+  }
   if (own) {
     cudaEventRecord(ev, work);
     cudaStreamWaitEvent(user, ev, 0);

@@ -83,6 +83,16 @@ int block_wait_status(exfem_block_s* b, cudaStream_t s) {
   return EXFEM_ERR_TIMEOUT;
 }
 
+// the same over every block of a solver: all flags are read and cleared
+static int solver_wait_status(exfem_solver_s* S, cudaStream_t s) {
+  int st = block_wait_status(S->blk, s);
+  for (auto* b : S->more) {
+    const int w = block_wait_status(b, s);
+    if (!st) st = w;
+  }
+  return st;
+}
+
 static int set_material(exfem_block_s* b, const exfem_material* m) {
   EX_ARG(m, "material is NULL");
   EX_ARG(m->kind == EXFEM_LINEAR_ELASTIC || m->kind == EXFEM_J2, "unknown material kind %d", m->kind);
@@ -576,7 +586,10 @@ int exfem_multi_pcg(exfem_block b, const double* Ke, int nrhs, const double* B, 
   StreamGuard g;
   int s;
   if ((s = g.init(stream))) return s;
-  return multi_pcg(b, Ke, nrhs, B, X, tol, maxiter, iters, relres, g.work);
+  const int r = multi_pcg(b, Ke, nrhs, B, X, tol, maxiter, iters, relres, g.work);
+  if (r < 0) return r;
+  const int w = block_wait_status(b, g.work);
+  return w < 0 ? w : r;
 }
 
 int exfem_ebe_matvec(exfem_block b, const double* Ke, const double* v, double* y, int apply_bc, void* stream) {
@@ -796,7 +809,7 @@ int exfem_solver_pcg(exfem_solver s, const double* b, double* x, double tol, int
   if ((st = g.init(stream))) return st;
   const int r = solver_pcg(s, b, x, tol, maxiter, iters, relres, g.work);
   if (r < 0) return r;
-  const int w = block_wait_status(s->blk, g.work);
+  const int w = solver_wait_status(s, g.work);
   return w < 0 ? w : r;
 }
 
@@ -816,7 +829,7 @@ int exfem_solver_mixed(exfem_solver s, const double* b, double* x, double tol, d
                                              relres, g.work))
                     : solver_mixed(s, b, x, tol, inner_tol, max_pass, maxiter, iters, passes, relres, g.work);
   if (r < 0) return r;
-  const int w = block_wait_status(s->blk, g.work);
+  const int w = solver_wait_status(s, g.work);
   return w < 0 ? w : r;
 }
 
@@ -834,7 +847,7 @@ int exfem_newton_increment(exfem_solver s, const double* u, const double* const*
   const int r = newton_increment(s, u, states_old, fext, start, rtol, max_iter, line_search != 0, cg_tol, cg_maxiter,
                                  qref, u_out, states_out, corrections, converged, ratios, lin_stats, g.work);
   if (r < 0) return r;
-  const int w = block_wait_status(s->blk, g.work);
+  const int w = solver_wait_status(s, g.work);
   return w < 0 ? w : r;
 }
 
@@ -952,6 +965,12 @@ int exfem_selftest_bounded_wait(int polls, void* stream) {
     return EXFEM_ERR_TIMEOUT;
   }
   return EXFEM_OK;
+}
+
+int exfem_selftest_block_wait(exfem_block b, int polls, void* stream) {
+  EX_ARG(b, "block is NULL");
+  EX_ARG(polls > 0, "polls must be positive");
+  return launch_wait_selftest(polls, b->dev_err.p, as_stream(stream));
 }
 
 // ---------------------------------------------------------------- host builders

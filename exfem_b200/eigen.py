@@ -22,6 +22,7 @@ import numpy as np
 import torch
 
 from . import linalg
+from ._lib import check, lib, stream_ptr
 from .solvers import State, _Setup
 
 _A, _B = 0.5854101966249685, 0.1381966011250105
@@ -138,6 +139,13 @@ def lobpcg(A, B, T, X0, k, tol=1e-6, maxiter=500, log=None):
     return np.asarray(lam[:k]), X[:, :k], it
 
 
+def _check_waits(blocks):
+    """Raise if a bounded device wait of the blocks' products gave up (the products
+    themselves return without synchronising)."""
+    for blk in blocks:
+        check(lib.exfem_block_status(blk.handle, stream_ptr()))
+
+
 def modal_lobpcg(model, step, nmodes, state=None, tol=1e-6, maxiter=500, log=None, operator="stored"):
     """(w^2 (nmodes,), modes (nmodes, ndof)) of a model under the step's prescribed
     DOFs (gfem/eigen.py:99-124; ``nmodes`` is the reference step's ``nmodes``); the
@@ -183,6 +191,7 @@ def modal_lobpcg(model, step, nmodes, state=None, tol=1e-6, maxiter=500, log=Non
     g = torch.Generator(device="cuda").manual_seed(0)
     X0 = torch.randn(nd, m, dtype=torch.float64, device="cuda", generator=g) * free[:, None]
     lam, V, it = lobpcg(A, B, T, X0, nmodes, tol=tol, maxiter=maxiter, log=log)
+    _check_waits(model.blocks)
     return np.maximum(lam, 0.0), V.T.contiguous()
 
 
@@ -227,6 +236,7 @@ def buckling_lobpcg(model, K0ops, KGops, setup, nmodes, monitor=None, tol=1e-6, 
     g = torch.Generator(device="cuda").manual_seed(1)
     X0 = torch.randn(model.ndof, m, dtype=torch.float64, device="cuda", generator=g) * free[:, None]
     mu, V, it = lobpcg(A, B, T, X0, nmodes, tol=tol, maxiter=maxiter, log=mon.log)
+    _check_waits([b for b, _ in K0ops + KGops])
     lam = np.where(mu < 0, -1.0 / np.where(mu < 0, mu, -1.0), np.inf)
     order = np.argsort(lam)
     mon.log(f"  LOBPCG converged in {it} iterations")
