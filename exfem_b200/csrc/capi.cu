@@ -338,8 +338,10 @@ int exfem_block_create(int etype, const exfem_material* mat, int64_t nn, const d
   if ((s = init_tangent(b.get()))) return s;
   // element-vector scratch (force assembly, stored-Ke products, diagonals); allocated
   // here so that no later call allocates inside a captured CUDA graph
-  // (twice where FP64 products need element vectors too: their own, so that a force
-  // evaluation and a solve of one block on two streams share nothing)
+  // (twice where the matrix-free FP64 products need element vectors too: theirs are apart
+  // from those of the forces, stored-Ke products and diagonals, as the tiles' partials of
+  // larger meshes are; calls that share a half, or a J2 block's tangent data, have to be
+  // ordered by their caller)
   if ((s = b->ys.alloc(std::max<int64_t>(ne * b->nnode * 3 * (product_by_points(etype, ne) ? 2 : 1), 1)))) return s;
   *out = b.release();
   return EXFEM_OK;

@@ -14,7 +14,9 @@
  *     stream; work is stream ordered and calls return without a device sync
  *     unless they must read a device scalar (solvers, which say so);
  *   - handles (block, amg, solver) own their device memory and are not thread
- *     safe: one host thread per handle;
+ *     safe: one host thread per handle; calls on one block share its scratch and a
+ *     J2 block's tangent data, so calls on different streams have to be ordered by
+ *     the caller (a solver's calls count as calls on its blocks and hierarchy);
  *   - DOF numbering is node-interleaved, dof = 3*node + component, as in the
  *     reference (gfem/model.py:157-158).
  */
