@@ -799,21 +799,20 @@ static int pcg_prepare(exfem_solver_s* S, cudaStream_t st) {
 }
 
 // chunks of PCG iterations until the device "done" flag is set (at most maxiter
-// iterations); the scalars are left in S->h_scal
+// iterations); the scalars are left in S->h_scal.  For the host-driven loop: with
+// device_loop the graph is a whole solve, launched by pcg_run, and the mixed solve is a
+// graph of its own.
 template <class T>
 static int pcg_chunks(exfem_solver_s* S, int maxiter, cudaStream_t st) {
   const int gi = sizeof(T) == 8 ? 0 : 1;
   const int chunk = S->chunk > 0 ? S->chunk : 8;
   int s;
-  // (a graph of the whole solve starts its own recursion: segments that continue one are
-  // launched kernel by kernel)
-  const bool graph = S->use_graph && !S->gloop[gi];
   const int max_chunks = maxiter / chunk + 2;
   for (int c = 0; c < max_chunks; ++c) {
     EX_CUDA(cudaMemcpyAsync(S->h_scal, S->scal.p, sizeof(PcgScal), cudaMemcpyDeviceToHost, st));
     EX_CUDA(cudaStreamSynchronize(st));
     if (S->h_scal->done) break;
-    if (graph) {
+    if (S->use_graph) {
       EX_CUDA(cudaGraphLaunch(S->gexec[gi], st));
     } else {
       for (int i = 0; i < chunk; ++i)
@@ -834,7 +833,7 @@ static int pcg_run(exfem_solver_s* S, double tol, int maxiter, int* iters, doubl
   init_scal_kernel<<<1, 1, 0, st>>>(S->scal.p, tol, maxiter);
   EX_LAUNCH_CHECK();
   const int gi = sizeof(T) == 8 ? 0 : 1;
-  if (S->use_graph && S->gexec[gi] && S->gloop[gi]) {  // one launch runs the solve to the end
+  if (S->use_graph && S->gloop[gi]) {  // one launch runs the solve to the end
     EX_CUDA(cudaGraphLaunch(S->gexec[gi], st));
     EX_CUDA(cudaMemcpyAsync(S->h_scal, S->scal.p, sizeof(PcgScal), cudaMemcpyDeviceToHost, st));
     EX_CUDA(cudaStreamSynchronize(st));
