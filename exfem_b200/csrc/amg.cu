@@ -287,7 +287,8 @@ static int bsr_launch(const Bsr& M, const T* val, const T* x, T* y, const T* b, 
     set_error("block-sparse product: misaligned operand (x %p, blocks %p)", (const void*)x, (const void*)val);
     return EXFEM_ERR_ARG;
   }
-  const double avg = M.nb ? (double)M.nnzb / (double)M.nb : 0.0;
+  if (M.nb == 0) return EXFEM_OK;  // a chained launch without rows would have a block that never waits
+  const double avg = (double)M.nnzb / (double)M.nb;
   // about two blocks per lane; rows of up to four blocks take single lanes once four
   // lanes a row would exceed the threads the chip holds (148 x 2,048): their blocks then
   // stream by (FP64 prolongation to 160,325 rows: 50 us less an iteration; to
