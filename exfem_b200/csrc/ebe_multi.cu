@@ -219,50 +219,68 @@ ebe_multi_kernel(int64_t ne, const int32_t* __restrict__ conn, const KT* __restr
   }
 }
 
-// Y[3n+c, r] = fixed ? V : sum over node n's gather-plan slots of the element rows,
-// the slots in the plan's order (slot s holds rows 3s .. 3s+2).  One thread per degree
-// of freedom and group of right-hand sides (four FP32, two FP64: 16 bytes) where their
-// number and the addresses allow it (vec), else one right-hand side; eight plan slots
-// and their rows are requested before any is added.  One thread per node, with three
-// rows of four slots in flight, took 23 us for 140,481 nodes and four FP32 right-hand
-// sides (18 us now).
-template <class VT, int W>
+// Y[3n+c, r] = fixed ? V : sum over node n's gather-plan slots of the element rows, the
+// slots in the plan's order (slot s holds rows 3s .. 3s+2).  One thread per RW rows (1 or
+// the node's 3) and NV groups of W right-hand sides (W = 16 bytes' worth where their number
+// and the addresses allow it, else 1); K plan slots and their values are requested before
+// any is added.  Bound by the latency of the plan -> row chain with few right-hand sides
+// and by the L1 pipe with many, where the plan's own reads count (once per thread).
+template <class VT, int W, int NV, int RW, int K>
 __global__ void __launch_bounds__(256)
-gather_multi_kernel(int64_t ndof, int vmax, const int32_t* __restrict__ plan, int32_t sentinel,
+gather_multi_kernel(int64_t nitem, int vmax, const int32_t* __restrict__ plan, int32_t sentinel,
                     const VT* __restrict__ ys, const uint8_t* __restrict__ fixed, const VT* __restrict__ V, int nrhs,
                     VT* __restrict__ Y) {
-  constexpr int K = 8;
   struct alignas(W * sizeof(VT)) Vec {
     VT v[W];
   };
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int nq = nrhs / W;
-  const int64_t d = nq == 1 ? t : t / nq;
-  if (d >= ndof) return;
-  const int r = (int)(t - d * nq) * W;
-  const int64_t n = d / 3;
+  const int nq = nrhs / (W * NV);
+  const int64_t item = nq == 1 ? t : t / nq;  // degree of freedom, or node (RW = 3)
+  if (item >= nitem) return;
+  const int r = (int)(t - item * nq) * (W * NV);
+  const int64_t n = RW == 3 ? item : item / 3, d = RW == 3 ? 3 * item : item;
   const int c = (int)(d - 3 * n);
   const int32_t* row = plan + n * vmax;
-  const bool pass = fixed && fixed[d];
-  Vec s;
+  Vec s[RW][NV];
 #pragma unroll
-  for (int j = 0; j < W; ++j) s.v[j] = VT(0);
+  for (int i = 0; i < RW; ++i)
+#pragma unroll
+    for (int h = 0; h < NV; ++h)
+#pragma unroll
+      for (int j = 0; j < W; ++j) s[i][h].v[j] = VT(0);
   for (int k0 = 0; k0 < vmax; k0 += K) {
     int32_t slot[K];
-    Vec w[K];
+    Vec w[K][RW][NV];
 #pragma unroll
     for (int k = 0; k < K; ++k) slot[k] = k0 + k < vmax ? row[k0 + k] : sentinel;
 #pragma unroll
     for (int k = 0; k < K; ++k)
-      if (slot[k] != sentinel) w[k] = *reinterpret_cast<const Vec*>(ys + (3 * (int64_t)slot[k] + c) * nrhs + r);
+      if (slot[k] != sentinel)
+#pragma unroll
+        for (int i = 0; i < RW; ++i)
+#pragma unroll
+          for (int h = 0; h < NV; ++h)
+            w[k][i][h] = reinterpret_cast<const Vec*>(ys + (3 * (int64_t)slot[k] + c + i) * nrhs + r)[h];
 #pragma unroll
     for (int k = 0; k < K; ++k)
       if (slot[k] != sentinel)
 #pragma unroll
-        for (int j = 0; j < W; ++j) s.v[j] += w[k].v[j];
+        for (int i = 0; i < RW; ++i)
+#pragma unroll
+          for (int h = 0; h < NV; ++h)
+#pragma unroll
+            for (int j = 0; j < W; ++j) s[i][h].v[j] += w[k][i][h].v[j];
     if (slot[K - 1] == sentinel) break;  // slots are listed without gaps
   }
-  *reinterpret_cast<Vec*>(Y + d * nrhs + r) = pass ? *reinterpret_cast<const Vec*>(V + d * nrhs + r) : s;
+#pragma unroll
+  for (int i = 0; i < RW; ++i) {
+    const bool pass = fixed && fixed[d + i];
+#pragma unroll
+    for (int h = 0; h < NV; ++h) {
+      const int64_t o = (d + i) * nrhs + r;
+      reinterpret_cast<Vec*>(Y + o)[h] = pass ? reinterpret_cast<const Vec*>(V + o)[h] : s[i][h];
+    }
+  }
 }
 
 template <class VT>
@@ -272,12 +290,24 @@ int launch_gather_multi(exfem_block_s* b, const VT* ys, const VT* V, VT* Y, int 
   const uint8_t* fx = bc ? b->fixed.p : nullptr;
   const int32_t sentinel = (int32_t)(b->ne * b->nnode);
   const bool vec = nrhs % W == 0 && ((uintptr_t)V | (uintptr_t)Y | (uintptr_t)ys) % 16 == 0;
-  const int64_t work = b->ndof() * (vec ? nrhs / W : nrhs);
-  const unsigned grid = (unsigned)((work + 255) / 256);
-  if (vec)
-    gather_multi_kernel<VT, W><<<grid, 256, 0, s>>>(b->ndof(), b->vmax, b->plan.p, sentinel, ys, fx, V, nrhs, Y);
-  else
-    gather_multi_kernel<VT, 1><<<grid, 256, 0, s>>>(b->ndof(), b->vmax, b->plan.p, sentinel, ys, fx, V, nrhs, Y);
+#define EXF_GATHER(W, NV, RW, K)                                                                                  \
+  do {                                                                                                            \
+    const int64_t nitem = RW == 3 ? b->nn : b->ndof(), work = nitem * (nrhs / (W * NV));                          \
+    gather_multi_kernel<VT, W, NV, RW, K><<<(unsigned)((work + 255) / 256), 256, 0, s>>>(nitem, b->vmax, b->plan.p, \
+                                                                                         sentinel, ys, fx, V, nrhs, Y); \
+  } while (0)
+  // B200, us with the rows cold, 256,000 C3D8 / 96,000 C3D10; in brackets one row and one
+  // group per thread with K = 8 for every count.  FP32: 4 right-hand sides 26 / 16, 8
+  // 41 / 23 (47 / 27), 12 55 / 32 (68 / 39), 16 67 / 35 (85 / 49); FP64: 8 67 / 36 (86 / 49),
+  // 16 126 / 65 (166 / 95).  Counts without 16-byte groups take a node's three rows per
+  // thread, which read the plan once: FP32 7 40 / 24 (72 / 44), FP64 15 126 / 72 (184 / 106);
+  // with one or two right-hand sides there is too little to read for that.
+  if (vec && nrhs % (2 * W) == 0) EXF_GATHER(W, 2, 1, 4);
+  else if (vec && nrhs > W) EXF_GATHER(W, 1, 1, 4);
+  else if (vec) EXF_GATHER(W, 1, 1, 8);
+  else if (nrhs >= 3) EXF_GATHER(1, 1, 3, 4);
+  else EXF_GATHER(1, 1, 1, (sizeof(VT) == 4 ? 4 : 8));
+#undef EXF_GATHER
   EX_LAUNCH_CHECK();
   return EXFEM_OK;
 }
