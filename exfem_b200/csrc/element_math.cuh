@@ -139,7 +139,7 @@ __host__ __device__ constexpr double tet10_dN(int g, int a, int i) {
 
 // ---------------------------------------------------------------- shape-function gradients
 // dN_b / dxi_i of the trilinear hexahedron at corner-ordered Gauss point g
-__host__ __device__ constexpr double hex_dN(int g, int b, int i) {
+__host__ __device__ __forceinline__ constexpr double hex_dN(int g, int b, int i) {
   const double p0 = HEX_GQ * hex_sign(g, 0), p1 = HEX_GQ * hex_sign(g, 1), p2 = HEX_GQ * hex_sign(g, 2);
   const double s0 = hex_sign(b, 0), s1 = hex_sign(b, 1), s2 = hex_sign(b, 2);
   const double f0 = 1.0 + s0 * p0, f1 = 1.0 + s1 * p1, f2 = 1.0 + s2 * p2;
