@@ -2,7 +2,9 @@
 // produces, the tangent data alone, element-averaged stresses, and the element vectors
 // of the FP64 tangent product (gfem/model.py:35-81, 129-137, 466-490).
 //
-// One warp takes 32 / ngp elements (4 C3D8, 8 C3D10), one lane per Gauss point.  Node
+// One warp takes 32 / ngp elements (4 C3D8, 8 C3D10), one lane per Gauss point (elastic
+// stresses and the elastic forces of larger C3D8 meshes one thread per element:
+// elastic_kernel).  Node
 // values are gathered once per element and Gauss-point states in whole lines into the
 // warp's shared memory; a lane evaluates its point's kinematics and material; the
 // element forces
@@ -43,6 +45,28 @@ struct ForceSmem {
   double c0[BBAR ? EPW : 1][9];  // mean stress times the inverse Jacobian of the centre
   uint64_t bar;                  // arrival of the states
 };
+
+// an element's stress output from the volume sums of its points (any of S, mises, peeq may
+// be NULL)
+template <int N>
+__device__ __forceinline__ void store_stress(int64_t e, const double (&sum)[N], double vol, double vol_alpha,
+                                             double* __restrict__ S, double* __restrict__ mises,
+                                             double* __restrict__ peeq) {
+  double s[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) s[k] = sum[k] / vol;
+  if (S) {
+    double* o = S + e * 9;
+    o[0] = s[0]; o[1] = s[3]; o[2] = s[5];
+    o[3] = s[3]; o[4] = s[1]; o[5] = s[4];
+    o[6] = s[5]; o[7] = s[4]; o[8] = s[2];
+  }
+  const double m3 = (s[0] + s[1] + s[2]) / 3.0;
+  const double d0 = s[0] - m3, d1 = s[1] - m3, d2 = s[2] - m3;
+  if (mises)
+    mises[e] = sqrt(1.5 * (d0 * d0 + d1 * d1 + d2 * d2 + 2.0 * (s[3] * s[3] + s[4] * s[4] + s[5] * s[5])));
+  if (peeq) peeq[e] = vol_alpha / vol;
+}
 
 // warps an SM holds: the products need few enough registers for 20, except the J2 C3D8's,
 // which would spill (126,000 elements: 80 us at 16, 111 us at 20)
@@ -191,20 +215,7 @@ force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict
 #pragma unroll
       for (int o = NG / 2; o > 0; o >>= 1) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
     if (valid && g == 0) {
-      double s[6];
-#pragma unroll
-      for (int k = 0; k < 6; ++k) s[k] = a[k] / a[6];
-      if (S) {
-        double* o = S + (int64_t)eid * 9;
-        o[0] = s[0]; o[1] = s[3]; o[2] = s[5];
-        o[3] = s[3]; o[4] = s[1]; o[5] = s[4];
-        o[6] = s[5]; o[7] = s[4]; o[8] = s[2];
-      }
-      const double m3 = (s[0] + s[1] + s[2]) / 3.0;
-      const double d0 = s[0] - m3, d1 = s[1] - m3, d2 = s[2] - m3;
-      if (mises)
-        mises[eid] = sqrt(1.5 * (d0 * d0 + d1 * d1 + d2 * d2 + 2.0 * (s[3] * s[3] + s[4] * s[4] + s[5] * s[5])));
-      if (peeq) peeq[eid] = J2 ? a[7] / a[6] : 0.0 / a[6];
+      store_stress(eid, a, a[6], a[7], S, mises, peeq);
     }
   }
 
@@ -304,6 +315,139 @@ force_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict
   }
 }
 
+// Elastic stresses, and elastic forces of C3D8 meshes that fill the chip: one thread per
+// element.  An elastic point has no state and little arithmetic, so the warp's transforms,
+// node values in shared memory and sums over an element's points are most of force_kernel's
+// time there; a thread that takes its element's points one after the other has none of them.
+// B200, us a call, warp / thread: stresses 40,000 C3D8 16.7 / 12.5, 432,000 142 / 58, 125,550
+// C3D10 37 / 23, 1,080,000 316 / 156 (equal up to some 10,000 elements, where a call is
+// its launch); C3D8 forces with the node sums 40,000 24.5 / 20.7, 128,000 63 / 41, 432,000
+// 218 / 129.
+template <int ET, int MODE>
+__global__ void __launch_bounds__(128)
+elastic_kernel(int64_t ne, const double* __restrict__ X, const int32_t* __restrict__ conn,
+               const double* __restrict__ u, const double* __restrict__ scale, const double* __restrict__ st_old,
+               double* __restrict__ st_new, double* __restrict__ fe, double* __restrict__ S,
+               double* __restrict__ mises, double* __restrict__ peeq, double lam_m, double mu_m,
+               const double* __restrict__ lam_e, const double* __restrict__ mu_e) {
+  constexpr int NN = ElemTraits<ET>::nnode, NG = ElemTraits<ET>::ngp;
+  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (e >= ne) return;
+  const double lam = lam_e ? lam_e[e] : lam_m, mu = lam_e ? mu_e[e] : mu_m;
+  int32_t nod[NN];
+#pragma unroll
+  for (int a = 0; a < NN; ++a) nod[a] = conn[e * NN + a];
+  double acc[6] = {0, 0, 0, 0, 0, 0}, vsum = 0.0;
+  if constexpr (ET == EXFEM_C3D8) {
+    const double sc = MODE == FORCE_FULL && scale ? scale[e] : 1.0;
+    double cm[7][3], um[7][3];
+    {
+      double xa[8][3], ua[8][3];
+#pragma unroll
+      for (int a = 0; a < 8; ++a)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          xa[a][c] = X[3 * (int64_t)nod[a] + c];
+          ua[a][c] = u[3 * (int64_t)nod[a] + c];
+        }
+#pragma unroll
+      for (int a = 7; a >= 0; --a)  // relative to the first node, as in gather_nodes
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          xa[a][c] -= xa[0][c];
+          ua[a][c] -= ua[0][c];
+        }
+      hex_to_modal(xa, cm);
+      hex_to_modal(ua, um);
+    }
+    double J0[9], iJ0[9], tr0 = 0.0, Fm[7][3], tacc = 0.0;
+#pragma unroll
+    for (int n = 0; n < 3; ++n)
+#pragma unroll
+      for (int i = 0; i < 3; ++i) J0[3 * n + i] = cm[i][n];
+    inv3(J0, iJ0);
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int i = 0; i < 3; ++i) tr0 += um[i][c] * iJ0[3 * i + c];
+#pragma unroll
+    for (int k = 0; k < 7; ++k) Fm[k][0] = Fm[k][1] = Fm[k][2] = 0.0;
+#pragma unroll 1
+    for (int g = 0; g < NG; ++g) {
+      const double x = HEX_GQ * hex_sign(g, 0), y = HEX_GQ * hex_sign(g, 1), z = HEX_GQ * hex_sign(g, 2);
+      double J[9], iJ[9], G[9], H[9], eps[6], sig[6];
+      hex_modal_grad(cm, x, y, z, J);
+      const double detJ = inv3(J, iJ);
+      hex_modal_grad(um, x, y, z, G);
+      matmul3(G, iJ, H);
+      const double bb = (tr0 - (H[0] + H[4] + H[8])) * (1.0 / 3.0);
+      H[0] += bb;
+      H[4] += bb;
+      H[8] += bb;
+      sym_from_grad(H, eps);
+      elastic_stress(lam, mu, eps, sig);
+      if constexpr (MODE == FORCE_STRESS) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) acc[k] += detJ * sig[k];
+        vsum += detJ;
+      } else {
+        const double vol = detJ * sc, t = vol * (sig[0] + sig[1] + sig[2]) * (1.0 / 3.0);
+        tacc += t;
+        const double r[3][3] = {{vol * sig[0] - t, vol * sig[3], vol * sig[5]},
+                                {vol * sig[3], vol * sig[1] - t, vol * sig[4]},
+                                {vol * sig[5], vol * sig[4], vol * sig[2] - t}};
+        double Q[9];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+            Q[3 * c + i] = r[c][0] * iJ[3 * i] + r[c][1] * iJ[3 * i + 1] + r[c][2] * iJ[3 * i + 2];
+        hex_modal_grad_adj(Q, x, y, z, Fm);
+        if (st_new) st_new[e * NG + g] = st_old ? st_old[e * NG + g] : 0.0;
+      }
+    }
+    if constexpr (MODE == FORCE_FULL) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) Fm[i][c] += tacc * iJ0[3 * i + c];
+      double f[8][3];
+      hex_from_modal(Fm, f);
+#pragma unroll
+      for (int a = 0; a < 8; ++a)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) fe[(e * 8 + a) * 3 + c] = f[a][c];
+    }
+  } else {
+    static_assert(MODE == FORCE_STRESS, "C3D10 forces are taken by force_kernel at every size");
+#pragma unroll 1
+    for (int g = 0; g < NG; ++g) {
+      double J[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, G[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, iJ[9], H[9], eps[6], sig[6];
+#pragma unroll
+      for (int a = 0; a < NN; ++a) {
+        const int64_t n3 = 3 * (int64_t)nod[a];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const double dn = elem_dN(ET, g, a, i);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            J[3 * c + i] += X[n3 + c] * dn;
+            G[3 * c + i] += u[n3 + c] * dn;
+          }
+        }
+      }
+      const double w = inv3(J, iJ) * (1.0 / 24.0);
+      matmul3(G, iJ, H);
+      sym_from_grad(H, eps);
+      elastic_stress(lam, mu, eps, sig);
+#pragma unroll
+      for (int k = 0; k < 6; ++k) acc[k] += w * sig[k];
+      vsum += w;
+    }
+  }
+  if constexpr (MODE == FORCE_STRESS) store_stress(e, acc, vsum, 0.0, S, mises, peeq);
+}
+
 template <int ET, bool J2, int MODE>
 int force_go(exfem_block_s* b, const double* u, const double* st_old, double* st_new, double* fe, double* S,
              double* mises, double* peeq, cudaStream_t s, const uint8_t* nf = nullptr, const int* skip = nullptr) {
@@ -329,6 +473,21 @@ int force_go(exfem_block_s* b, const double* u, const double* st_old, double* st
   return EXFEM_OK;
 }
 
+template <int ET, int MODE>
+int elastic_go(exfem_block_s* b, const double* u, const double* st_old, double* st_new, double* fe, double* S,
+               double* mises, double* peeq, cudaStream_t s) {
+  elastic_kernel<ET, MODE><<<(unsigned)((b->ne + 127) / 128), 128, 0, s>>>(
+      b->ne, b->X.p, b->conn.p, u, b->scale.p, st_old, st_new, fe, S, mises, peeq, b->mat.lam, b->mat.mu, b->lam_e.p,
+      b->mu_e.p);
+  EX_LAUNCH_CHECK();
+  return EXFEM_OK;
+}
+
+// a thread takes eight times as long over its element as the lanes of a warp, and its blocks
+// cover the chip from some 19,000 elements on (148 x 128); forces, us a call, warp / thread:
+// 4,000 elements 8.5 / 11.1, 8,000 10.4 / 12.5, 12,000 12.5 / 12.5, 16,000 14.5 / 12.5
+bool elastic_force_by_threads(int64_t ne) { return ne > 12000; }
+
 template <int ET>
 int force_et(exfem_block_s* b, int mode, const double* u, const double* st_old, double* st_new, double* fe, double* S,
              double* mises, double* peeq, cudaStream_t s) {
@@ -337,9 +496,11 @@ int force_et(exfem_block_s* b, int mode, const double* u, const double* st_old, 
     if (mode == FORCE_TANGENT) return force_go<ET, true, FORCE_TANGENT>(b, u, st_old, st_new, fe, S, mises, peeq, s);
     return force_go<ET, true, FORCE_STRESS>(b, u, st_old, st_new, fe, S, mises, peeq, s);
   }
-  if (mode == FORCE_FULL) return force_go<ET, false, FORCE_FULL>(b, u, st_old, st_new, fe, S, mises, peeq, s);
   if (mode == FORCE_TANGENT) return EXFEM_OK;  // an elastic tangent does not change
-  return force_go<ET, false, FORCE_STRESS>(b, u, st_old, st_new, fe, S, mises, peeq, s);
+  if (mode == FORCE_STRESS) return elastic_go<ET, FORCE_STRESS>(b, u, st_old, st_new, fe, S, mises, peeq, s);
+  if constexpr (ET == EXFEM_C3D8)
+    if (elastic_force_by_threads(b->ne)) return elastic_go<ET, FORCE_FULL>(b, u, st_old, st_new, fe, S, mises, peeq, s);
+  return force_go<ET, false, FORCE_FULL>(b, u, st_old, st_new, fe, S, mises, peeq, s);
 }
 
 }  // namespace
