@@ -4,10 +4,9 @@
 //
 // One warp takes 32 / ngp elements (4 C3D8, 8 C3D10), one lane per Gauss point (elastic
 // stresses and the elastic forces of larger C3D8 meshes one thread per element:
-// elastic_kernel).  Node
-// values are gathered once per element and Gauss-point states in whole lines into the
-// warp's shared memory; a lane evaluates its point's kinematics and material; the
-// element forces
+// elastic_kernel).  Node values are gathered once per element and Gauss-point states in
+// whole lines into the warp's shared memory; a lane evaluates its point's kinematics and
+// material; the element forces
 //   f_a = sum_g sum_i dN_a/dxi_i(g) Q_g[:, i],  Q_g = vol sigma J^-T,
 // are one small product of the constant dN table with the Q of all the warp's elements
 // side by side, done with the FP64 matrix instruction, which also sums over the lanes;
@@ -68,8 +67,9 @@ __device__ __forceinline__ void store_stress(int64_t e, const double (&sum)[N], 
   if (peeq) peeq[e] = vol_alpha / vol;
 }
 
-// warps an SM holds: the products need few enough registers for 20, except the J2 C3D8's,
-// which would spill (126,000 elements: 80 us at 16, 111 us at 20)
+// warps an SM holds: the products need few enough registers for 20 (with the node sums, 16
+// and 20 warps: 116,000 C3D8 55.2 / 53.2 us, 329,232 C3D10 125 / 116), except the J2 C3D8's,
+// which spill (116,000 elements 73.4 / 76.7)
 template <int ET, bool J2, int MODE>
 constexpr int force_warps() {
   return MODE == FORCE_PRODUCT && !(J2 && ET == EXFEM_C3D8) ? 20 : 16;

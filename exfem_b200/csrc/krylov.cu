@@ -3,7 +3,8 @@
 // PCG follows gfem/linalg.py:21-47 exactly: x0 = 0, r = b, z = M(r), p = z,
 // loop while r.r > tol^2 max(b.b, 1e-300) and k < maxiter: Ap = A p,
 // alpha = rz / p.Ap, x += alpha p, r -= alpha Ap, rr = r.r, z = M(r),
-// beta = r.z / rz, p = z + beta p.  All dot products accumulate in FP64 with a
+// beta = r.z / rz, p = z + beta p (FP32 recursions take the conjugacy form of beta where
+// r.z rises or changes sign: pcg_iteration).  All dot products accumulate in FP64 with a
 // fixed two-level reduction order (deterministic), and all step scalars live in
 // device memory as FP64, so the host never sits in the loop: iterations are
 // issued in chunks (captured once as a CUDA graph), every kernel first reads the

@@ -61,8 +61,8 @@ struct StiffSmem {
 // shared memory and leaves as one bulk store, so that global memory sees whole lines.
 // MODE 1 writes the diagonal entries only.
 //
-// Measured on B200: 40,000 J2 C3D8 (184 MB of Ke) 66 us, 72,450 C3D10 (522 MB) 109 us
-// = 0.75 of the copy bandwidth; one thread per node, which formed every gradient again
+// Measured on B200: 40,000 J2 C3D8 (184 MB of Ke) 64 us, 72,450 C3D10 (522 MB) 109 us
+// = 0.73 of the copy bandwidth; one thread per node, which formed every gradient again
 // for each node pair and stored single entries, took 1,273 and 1,418 us.  C3D10 is
 // bound by the stores; C3D8 by the latency of the material phase at 12 warps an SM:
 // four blocks' worth of registers (128 a thread) spill there and take 88 us, two take
