@@ -3,8 +3,8 @@
 // PCG follows gfem/linalg.py:21-47 exactly: x0 = 0, r = b, z = M(r), p = z,
 // loop while r.r > tol^2 max(b.b, 1e-300) and k < maxiter: Ap = A p,
 // alpha = rz / p.Ap, x += alpha p, r -= alpha Ap, rr = r.r, z = M(r),
-// beta = r.z / rz, p = z + beta p (FP32 recursions take the conjugacy form of beta where
-// r.z rises or changes sign: pcg_iteration).  All dot products accumulate in FP64 with a
+// beta = r.z / rz, p = z + beta p (FP32 recursions with a V-cycle take the conjugacy form
+// of beta where r.z rises or changes sign: pcg_iteration).  All dot products accumulate in FP64 with a
 // fixed two-level reduction order (deterministic), and all step scalars live in
 // device memory as FP64, so the host never sits in the loop: iterations are
 // issued in chunks (captured once as a CUDA graph), every kernel first reads the
@@ -540,16 +540,19 @@ static int pc_apply(exfem_solver_s* S, const T* r, T* z, const int* skip, cudaSt
 // some 35 kernels an iteration).
 //
 // beta = r.z / (r.z)_old and -z.Ap / p.Ap are the same number in exact arithmetic.  The
-// FP32 recursion takes the second, which makes the new direction conjugate to the last one
-// as the product has it, where the first lies outside [0, 1]: the V-cycle is indefinite on
-// some vectors of a mesh with strongly varying moduli, r.z passes through zero there, and
-// dividing by it gives directions (beta 62 was met) that hold little but rounding.  Inside
-// [0, 1] r.z falls as it should and the first is the better determined one: after a large
-// drop z.Ap is a small difference of large terms (on a mesh with an exact preconditioner it
-// led to non-finite steps).  C3D10 cubes with moduli over a decade, cg_tol 1e-8, FP32
-// iterations with the first form alone and now: 12.5M DOF, five seeds, 131 201 82 152 104
-// and 93 116 82 138 95; 1.6M DOF, four seeds, 102 69 63 64 and 78 70 61 62; where r.z never
-// rises the iterates are the same.
+// FP32 recursion with a V-cycle takes the second, which makes the new direction conjugate
+// to the last one as the product has it, where the first lies outside [0, 1]: the V-cycle is
+// indefinite on some vectors of a mesh with strongly varying moduli, r.z passes through zero
+// there, and dividing by it gives directions (beta 62 was met) that hold little but
+// rounding.  Inside [0, 1] r.z falls as it should and the first is the better determined
+// one: after a large drop z.Ap is a small difference of large terms (on a mesh with an exact
+// preconditioner it led to non-finite steps).  C3D10 cubes with moduli over a decade, cg_tol
+// 1e-8, FP32 iterations with the first form alone and now: 12.5M DOF, five seeds, 131 201 82
+// 152 104 and 93 116 82 138 95; 1.6M DOF, four seeds, 102 69 63 64 and 78 70 61 62; where
+// r.z never rises the iterates are the same.  The diagonal and polynomial preconditioners are
+// positive definite, their r.z rises often and harmlessly, and the kept directions of
+// replaced residuals are better served by the first form (mixed Jacobi solves of 320 to 1,536
+// elements took up to a quarter more iterations with the second).
 template <class T>
 static int pcg_iteration(exfem_solver_s* S, cudaStream_t st, bool looped) {
   const int* skip = looped ? nullptr : &S->scal.p->done;
@@ -561,7 +564,7 @@ static int pcg_iteration(exfem_solver_s* S, cudaStream_t st, bool looped) {
                  S->scal.p);
   EX_LAUNCH_CHECK();
   if ((s = pc_apply<T>(S, r, z, skip, st))) return s;
-  if constexpr (sizeof(T) == 8) {
+  if (sizeof(T) == 8 || S->pc != EXFEM_PC_AMG) {
     if ((s = dot<T>(S, r, z, FIN_BETA, nullptr, 1, st))) return s;
   } else {
     launch_chained(dot_conj_kernel<T>, red_grid(S->n), RT, 0, st, S->n, z, r, Ap, S->partial.p, S->counter.p, S->scal.p);

@@ -358,7 +358,8 @@ int exfem_solver_set_graph(exfem_solver s, int enable, int chunk);
 int exfem_solver_set_loop(exfem_solver s, int device_loop);
 /* PCG in the operator's precision with FP64 scalars and dot products
  * (gfem/linalg.py:21-47): x0 = 0, stop when r.r <= tol^2 b.b or k >= maxiter.  FP32
- * recursions take beta = -z.Ap / p.Ap where r.z / (r.z)_old lies outside [0, 1].
+ * recursions with EXFEM_PC_AMG take beta = -z.Ap / p.Ap where r.z / (r.z)_old lies
+ * outside [0, 1].
  * b, x: FP64 device (ndof).  Synchronises the stream to read the iteration count.
  * Returns EXFEM_NOT_CONVERGED when relres > 1e-3 or is not finite (the
  * reference's warning condition, gfem/solvers.py:472-473). */
